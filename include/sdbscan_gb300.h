@@ -117,11 +117,12 @@ sdb_status sdb_set_precision(sdb_engine* e, int32_t precision);
 sdb_status sdb_set_debug_limits(sdb_engine* e, int64_t stall_spins, int64_t queue_cap, int64_t device_bytes_cap);
 
 /* Tile shape of the plain FP32 distance kernel (a tuning control; no
- * reference counterpart): 0 = by topM and distance (default: for topM in
- * 41..50 shape 3 with Cosine, shape 2 otherwise; else 1), 1 = 128 x 64 tiles on 256 threads, 2 = 128 x 50 on 160 threads
- * (32 dimensions per stage, 2 stages), 3 = 128 x 50 with 16 dimensions per
- * stage in 4 stages (Cosine; shape 2 for the other distances), 4 and 5 = the
- * persistent warp-specialised kernel (a producer warp gathers the rows, the
+ * reference counterpart): 0 = the default: shape 3 where the distance has it
+ * (Cosine, L1, L2) and the lists have 16 members or more on average, else 2 for topM in 41..50 and 1 otherwise, 1 = 128 x 64
+ * tiles on 256 threads, 2 = 128 x 50 on 160 threads (32 dimensions per stage, 2
+ * stages), 3 = the packed tile (two columns per instruction; 32, 40, 50 or 64
+ * columns by topM; it keeps a copy of the candidate rows, and where that does
+ * not fit in memory the scalar shapes run instead), 4 and 5 = the persistent warp-specialised kernel (a producer warp gathers the rows, the
  * other warps compute; 4 stages and 3 CTAs per SM, or 6 stages and 2).  The
  * 50-column shapes apply when topM <= 50 (else the 64-column ones).  Any shape
  * gives the same bits. */

@@ -50,51 +50,6 @@ SDB_DEV int warp_sum(int v) {
     return v;
 }
 
-// Calls f(i) on the warp's lanes for every candidate i of point p that passed
-// eps (bit set in p's mask words).  The 2k top-k ids and mask words are
-// fetched up front, two slots per lane; candidates come in lane-parallel
-// batches of up to 32.
-template <typename F>
-SDB_DEV void for_each_passing(const int32_t* __restrict__ topK, const int32_t* __restrict__ topM,
-                              const uint64_t* __restrict__ masks, int k, int m, int W, int p, F&& f) {
-    const unsigned l = lane_id();
-    const int slots = 2 * k;
-    const unsigned long long* mk64 = reinterpret_cast<const unsigned long long*>(masks);
-    int rA = 0, rB = 0;
-    uint64_t mA = 0, mB = 0;
-    if ((int)l < slots) {
-        rA = __ldg(topK + (size_t)p * slots + l);
-        mA = __ldg(mk64 + ((size_t)p * slots + l) * W);
-    }
-    if ((int)l + 32 < slots) {
-        rB = __ldg(topK + (size_t)p * slots + l + 32);
-        mB = __ldg(mk64 + ((size_t)p * slots + l + 32) * W);
-    }
-    for (int jj = 0; jj < slots; ++jj) {
-        const int src = jj & 31;
-        const int r = __shfl_sync(0xffffffffu, jj < 32 ? rA : rB, src);
-        const int side = jj >= k;
-        const int32_t* lst = topM + (size_t)r * 2 * m + side * m;
-        for (int wd = 0; wd < W; ++wd) {
-            uint64_t mk;
-            if (wd == 0) {
-                const uint64_t mine = jj < 32 ? mA : mB;
-                const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)mine, src);
-                const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(mine >> 32), src);
-                mk = ((uint64_t)hi << 32) | lo;
-            } else {
-                mk = __ldg(mk64 + ((size_t)p * slots + jj) * W + wd);
-            }
-            if (!mk) continue;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int bit = half * 32 + (int)l;
-                if ((mk >> bit) & 1ull) f(__ldg(lst + wd * 64 + bit));
-            }
-        }
-    }
-}
-
 // Distance codes (sdb_distance in include/sdbscan_gb300.h).
 enum { DIST_COSINE = 0, DIST_L1 = 1, DIST_L2 = 2, DIST_CHI2 = 3, DIST_JS = 4 };
 
@@ -250,8 +205,10 @@ struct DistArgs {
     const int64_t* tileTotal;  // device: actual number of tiles
     const int32_t* tilePerm;   // optional: launch order of the tiles (tile_at)
     const int32_t* topM;
-    int nproj, m, k, W;   // W = 64-bit mask words per (point, slot)
-    int nct;              // candidate tiles per list
+    int nproj, m, k, W;   // W = 64-bit mask words per (point, slot), one per candidate tile
+    int nct;              // candidate tiles per list (= W)
+    int TM, CT;           // member rows and candidate columns per tile: bit j of word w is column CT w + j
+    float* cand;          // packed tile: the lists' candidate rows, dimension-major (launch_cand_tiles), or null
     float eps;
     float epsLo;          // eps sweeps: k_masks_from_dists keeps epsLo < d <= eps
     const uint8_t* pairRound;  // eps sweeps (optional): per pair, the first round whose eps >= d (rows of W x 64 bytes)
@@ -271,6 +228,14 @@ struct DistArgs {
 };
 constexpr int kMaxScreenedSweep = 16;
 int launch_dist(const DistArgs& a, cudaStream_t st);
+// The packed tile (pair_tile.cuh): candidate columns per tile for a distance
+// and topM (0: this distance has none), its member rows, the bytes of the
+// candidate copy, the copy's kernel and the distance kernel.
+int pair_tile_cols(int dist, int m);
+int pair_tile_rows(int cols);
+size_t pair_cand_bytes(int cols, int nproj, int m, int ld);
+int launch_cand_tiles(const DistArgs& a, cudaStream_t st);
+int launch_dist_pair(const DistArgs& a, cudaStream_t st);
 // The persistent warp-specialised plain kernel (k_dist_ws.cu): variant 4 or 5.
 int launch_dist_ws(const DistArgs& a, int variant, cudaStream_t st);
 int launch_masks_from_dists(const DistArgs& a, cudaStream_t st);
@@ -294,6 +259,7 @@ int launch_recheck(const DistArgs& a, const uint64_t* queue, const unsigned long
 
 struct CoreArgs {
     int n, k, m, W, nproj, minPts;
+    int CT;               // candidate columns per mask word
     const uint64_t* masks;
     const int32_t* topK;
     const int32_t* topM;
@@ -319,7 +285,7 @@ struct CoreArgs {
 };
 // Per-slot signatures (sig, 2D x m int4) and the multi-list slot bits (multi, 2D x W).
 int launch_slot_sigs(const int32_t* topM, int D, int m, const int64_t* hubOff, const int32_t* hubLists, void* sig,
-                     uint64_t* multi, int W, cudaStream_t st);
+                     uint64_t* multi, int W, int CT, cudaStream_t st);
 int launch_core_dedupe(const CoreArgs& a, const void* sig, cudaStream_t st);
 // hubIdx from hubOff (a scan of hub flags into idxTmp) and the hubs' list masks.
 int launch_hub_masks(const CoreArgs& a, int32_t* hubIdx, int64_t* idxTmp, uint32_t* kMask, int64_t* scanTmp,
@@ -331,7 +297,7 @@ struct ClusterArgs {
     const uint64_t* masks;   // first-occurrence masks: each distinct candidate once per point
     const int32_t* topK;
     const int32_t* topM;
-    // the distance stage's tiles (list l, 128 member rows, 64 candidate columns)
+    // the distance stage's tiles (list l, TM member rows, CT candidate columns)
     const int2* members;
     const int64_t* listOff;
     const int32_t* tileList;
@@ -339,7 +305,7 @@ struct ClusterArgs {
     const int64_t* tileTotal;  // device: actual number of tiles
     const int32_t* tilePerm;   // optional: launch order of the tiles (tile_at)
     int64_t nTiles;            // launch grid (an upper bound)
-    int TM, nct, nproj;
+    int TM, CT, nct, nproj;
     // eps sweeps: the union-find carries over from the previous (smaller) eps,
     // and only rows with a new edge or a newly core endpoint are united
     int carry, round;

@@ -43,6 +43,12 @@ namespace {
 // Point chunks per super-chunk of the tensor-core distance kernel's tile order
 // (launch_tile_order_list), and the key count of that order's counting sort.
 constexpr int kSuperChunk = 8;
+
+// Largest candidate copy of the packed distance tile (1M x 784 with D = 1024
+// and m = 50 takes 0.33 GB).
+constexpr size_t kMaxCandBytes = (size_t)8 << 30;
+constexpr int kMinCandMembers = 16;
+
 size_t kTcKeys(int n, int L) {
     const int nChunks = (n + 4095) / 4096;
     return (size_t)((nChunks + kSuperChunk - 1) / kSuperChunk) * L + 1;
@@ -88,6 +94,13 @@ bool sdb_engine::ensure(DevBuf& b, size_t bytes) {
     return true;
 }
 
+void sdb_engine::release(DevBuf& b) {
+    if (b.ptr) cudaFree(b.ptr);
+    devBytes -= b.bytes;
+    b.ptr = nullptr;
+    b.bytes = 0;
+}
+
 sdb_status sdb_engine::fail(sdb_status s, const std::string& msg) {
     err = msg;
     return s;
@@ -115,7 +128,7 @@ std::vector<DevBuf*> sdb_engine::all_bufs() {
             &kMask, &firstMasks, &Xb, &queue, &sweepLabels, &sweepNcl, &sig, &Rb, &newMasks, &coreEps, &sampleFlag,
             &noiseFlag, &noiseCores, &noisePts, &PcT, &numCore, &pairRound, &sngCols, &sngMult, &sngColOf, &sngExtras,
             &sngExtraPass, &sngMask, &rowDeg, &colCnt, &sngUb, &sngHeavy, &chunkOff, &tileKey, &keyOff, &tilePerm,
-            &Cb, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask};
+            &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask};
 }
 
 // ---------------------------------------------------------------------------
@@ -190,6 +203,19 @@ void sdb_engine::host_random(int seedUsed) {
 // the fit pipeline
 // ---------------------------------------------------------------------------
 sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts, bool optics, const SweepSpec* sw) {
+    sdb_status s = fit_once(X, xOnDevice, eps, minPts, optics, sw);
+    // out of memory with the packed tile's candidate copy: once more without it
+    if (s == SDB_ERR_NOMEM && candT.ptr != nullptr && !(sw != nullptr && sw->capture)) {
+        cudaStreamSynchronize(stream);
+        release(candT);
+        noCandCopy = true;
+        s = fit_once(X, xOnDevice, eps, minPts, optics, sw);
+    }
+    return s;
+}
+
+sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int minPts, bool optics,
+                                const SweepSpec* sw) {
     if (!paramsSet) return fail(SDB_ERR_STATE, "set_params must be called before a fit");
     const bool sweep = sw != nullptr, capture = sw != nullptr && sw->capture;
     if (sweep && (optics || sw->nEps < 1 || !sw->eps || !sw->labelsDev || !sw->nclDev))
@@ -209,10 +235,6 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
     cudaError_t ce = cudaSetDevice(device);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaSetDevice");
 
-    const int TMr = dist_tile_rows(), TNc = dist_tile_cols();
-    const int nct = (m + TNc - 1) / TNc;
-    const int W = (m + 63) / 64;
-    const int L = 2 * D;
     // top-m threshold chunks: six chunks per projection block of one full
     // wave (project_wave_chunks), so the grid-stride blocks end together, and
     // at least 4m chunks so the chunk maxima bound the m-th value
@@ -221,7 +243,6 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
     const int G = (n + chunk - 1) / chunk;
     int cap = 256;
     while (cap < 8 * m) cap <<= 1;
-    const int64_t maxTiles = ((int64_t)n * 2 * k / TMr + L) * nct;
     const bool rff = p.distance == SDB_L1 || p.distance == SDB_L2;
     // BF16 tensor-core screening of the candidate distances: Cosine sDBSCAN
     // fits and eps sweeps of up to kMaxScreenedSweep values (the projection
@@ -231,6 +252,22 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
                         ((p.distance == SDB_COSINE && (!sweep || sw->nEps <= kMaxScreenedSweep)) ||
                          (p.distance == SDB_L2 && !sweep));
     const int ldb = (d + 63) / 64 * 64;
+    // the distance tiles: the packed tile where the distance has one (and no
+    // other shape is asked for), else 128 x 64.  It reads a copy of the lists'
+    // candidate rows; past kMaxCandBytes (wide data and many vectors) that
+    // copy costs more memory than a list's few tiles are worth, and below
+    // kMinCandMembers members per list it takes longer than the tiles save
+    // (2K x 64, k = 5, D = 1024, 10 members: 47 us with the copy, 43 without;
+    // 4K x 128, 20 members: 82 against 92; 50K x 128, 244: 232 against 309).
+    const bool wantPair = distVariant == 3 || (distVariant == 0 && (int64_t)n * k >= (int64_t)kMinCandMembers * D);
+    const int pairCols = screen || !wantPair ? 0 : pair_tile_cols(p.distance, m);
+    const bool pairTiles = pairCols > 0 && !noCandCopy && pair_cand_bytes(pairCols, D, m, ld) <= kMaxCandBytes &&
+                           ensure(candT, pair_cand_bytes(pairCols, D, m, ld));
+    const int TMr = pairTiles ? pair_tile_rows(pairCols) : dist_tile_rows();
+    const int CT = pairTiles ? pairCols : dist_tile_cols();
+    const int nct = (m + CT - 1) / CT, W = nct;
+    const int L = 2 * D;
+    const int64_t maxTiles = ((int64_t)n * 2 * k / TMr + L) * nct;
     const bool fuseXb = screen && p.distance == SDB_COSINE && fhtDim <= 2048 && ldb <= fhtDim;
 
     // allocations (grow-only)
@@ -451,7 +488,7 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
     SDB_CK(cudaMemsetAsync(hubCount.ptr, 0, sizeof(int32_t) * n, st));
     L_(launch_hubs_scatter(ia, st));
     L_(launch_slot_sigs(i32(topM), D, m, i64(hubOff), i32(hubLists), sig.ptr, static_cast<uint64_t*>(multiMask.ptr), W,
-                        st));
+                        CT, st));
     if (!ok) return fail(SDB_ERR_CUDA, std::string("index launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     if (!capture) SDB_CK(cudaEventRecord(ev[4], st));
 
@@ -475,6 +512,9 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
     da.k = k;
     da.W = W;
     da.nct = nct;
+    da.TM = TMr;
+    da.CT = CT;
+    da.cand = pairTiles ? f32(candT) : nullptr;
     da.eps = eps;
     if (sweep) da.eps = *std::max_element(sw->eps, sw->eps + sw->nEps);
     da.masks = static_cast<uint64_t*>(masks.ptr);
@@ -525,7 +565,12 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
         if (!ok) return fail(SDB_ERR_CUDA, std::string("tensor-core distance launch failed: ") +
                                                cudaGetErrorString(cudaGetLastError()));
     }
-    L_(launch_dist(da, st));
+    if (pairTiles) {
+        L_(launch_cand_tiles(da, st));
+        L_(launch_dist_pair(da, st));
+    } else {
+        L_(launch_dist(da, st));
+    }
     if (!ok) return fail(SDB_ERR_CUDA, std::string("distance launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     if (!capture) SDB_CK(cudaEventRecord(ev[5], st));
 
@@ -535,6 +580,7 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
     ca.k = k;
     ca.m = m;
     ca.W = W;
+    ca.CT = CT;
     ca.nproj = D;
     ca.minPts = minPts;
     ca.masks = static_cast<const uint64_t*>(masks.ptr);
@@ -614,6 +660,7 @@ sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts
         ka.tilePerm = i32(tilePerm);
         ka.nTiles = maxTiles;
         ka.TM = TMr;
+        ka.CT = CT;
         ka.nct = nct;
         ka.nproj = D;
         ka.core = static_cast<const uint8_t*>(core.ptr);

@@ -82,7 +82,7 @@ struct sdb_engine {
         rootFlag, labels, nClusters, scanTmp, errFlags, counters, E, Rt, signs, compCosh, dists, coreDist, nbOff,
         nbIdx, nbDist, nbFill, hubIdx, kMask, firstMasks, Xb, queue, sweepLabels, sweepNcl, sig, Rb, newMasks,
         coreEps, sampleFlag, noiseFlag, noiseCores, noisePts, PcT, numCore, pairRound, sngCols, sngMult, sngColOf,
-        sngExtras, sngExtraPass, sngMask, rowDeg, colCnt, sngUb, sngHeavy, chunkOff, tileKey, keyOff, tilePerm, Cb,
+        sngExtras, sngExtraPass, sngMask, rowDeg, colCnt, sngUb, sngHeavy, chunkOff, tileKey, keyOff, tilePerm, Cb, candT,
         tileKeyTc, keyOffTc, tilePermTc, sngWords, hashOffB, hashIdB, hashDistB, sqNorm, multiMask;
 
     // results
@@ -102,6 +102,7 @@ struct sdb_engine {
     int64_t fallbacks = 0;  // BF16 screening fits redone on the plain path
     int sngColsLast = 0, sngExtraLast = 0;  // sampled columns and extra draws of the last sng fit
     int distVariant = 0;    // plain distance tile shape (DistArgs::variant), set by the batch's autotuner
+    bool noCandCopy = false;  // the packed distance tile's candidate copy did not fit in memory
     int sngSampling = 0;    // sngDbscan sample: 0 = by seed (shared when >= 0, blocks when < 0), 1 = shared, 2 = blocks
     // test and diagnostic limits (sdb_set_debug_limits), 0 = off
     long long dbgStallSpins = 0;  // each tensor-core / persistent distance kernel takes its failure path once
@@ -111,6 +112,7 @@ struct sdb_engine {
     float stageMs[9] = {};
 
     bool ensure(DevBuf& b, size_t bytes);
+    void release(DevBuf& b);
     sdb_status fail(sdb_status s, const std::string& msg);
     sdb_status cuda_fail(cudaError_t e, const char* where);
     void free_all();
@@ -119,6 +121,7 @@ struct sdb_engine {
     void host_random(int seed);
     sdb_status fit(const float* X, bool xOnDevice, float eps, int minPts, bool optics,
                    const SweepSpec* sw = nullptr);
+    sdb_status fit_once(const float* X, bool xOnDevice, float eps, int minPts, bool optics, const SweepSpec* sw);
     sdb_status check_flags();
     sdb_status optics_stage(const sdb::CoreArgs& ca, int& launches);
     sdb_status optics_order(int64_t total);

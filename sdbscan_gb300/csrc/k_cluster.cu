@@ -26,7 +26,7 @@ __global__ void k_init(int32_t* parent, int32_t* border, int n, int keepParent) 
 }
 
 // A tile of the distance stage: list l's member rows [mbeg, mend) against its
-// candidate columns [64 ct, 64 ct + 64) (mask word ct).
+// candidate columns [CT ct, CT ct + CT) (mask word ct).
 struct Tile {
     int64_t mbeg, mend;
     int ct;
@@ -53,7 +53,7 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
 // unites only where they differ.  A cached value is always an ancestor of its
 // candidate (parents only move up), so equality proves the same set; a stale
 // value only costs a redundant unite.
-__global__ void __launch_bounds__(128) k_union_tiles(ClusterArgs a) {
+__global__ void __launch_bounds__(256) k_union_tiles(ClusterArgs a) {
     __shared__ int croot[64];
     __shared__ unsigned long long newCoreCand;  // carry: candidates that became core this round
     Tile tl;
@@ -63,8 +63,8 @@ __global__ void __launch_bounds__(128) k_union_tiles(ClusterArgs a) {
     __syncthreads();
     int q = -1;  // this thread's candidate (threads < 64)
     if (threadIdx.x < 64) {
-        const int c = tl.ct * 64 + threadIdx.x;
-        if (c < a.m) {
+        const int c = tl.ct * a.CT + threadIdx.x;
+        if ((int)threadIdx.x < a.CT && c < a.m) {
             q = __ldg(tl.cand + c);
             if (a.carry && a.core[q] && a.coreEps[q] == a.round) atomicOr(&newCoreCand, 1ull << threadIdx.x);
         }
@@ -111,13 +111,13 @@ __global__ void k_compress(ClusterArgs a) {
 // member takes the smallest root among its passing core candidates; a non-core
 // candidate takes the smallest root among the core members passing with it,
 // reduced in shared memory first so each candidate sees one global atomic.
-__global__ void __launch_bounds__(128) k_border_tiles(ClusterArgs a) {
+__global__ void __launch_bounds__(256) k_border_tiles(ClusterArgs a) {
     __shared__ int croot[64], cbest[64], cpt[64];
     Tile tl;
     if (!tile_of(a, blockIdx.x, tl)) return;
     if (threadIdx.x < 64) {
-        const int c = tl.ct * 64 + threadIdx.x;
-        const int q = c < a.m ? __ldg(tl.cand + c) : -1;
+        const int c = tl.ct * a.CT + threadIdx.x;
+        const int q = (int)threadIdx.x < a.CT && c < a.m ? __ldg(tl.cand + c) : -1;
         cpt[threadIdx.x] = q;
         croot[threadIdx.x] = (q >= 0 && a.core[q]) ? __ldcg(a.parent + q) : INT_MAX;
         cbest[threadIdx.x] = INT_MAX;
@@ -178,11 +178,11 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st) {
     const int g = (a.n + 255) / 256;
     k_init<<<g, 256, 0, st>>>(a.parent, a.border, a.n, a.carry && a.round > 0);
     ++launches;
-    k_union_tiles<<<(unsigned)a.nTiles, 128, 0, st>>>(a);
+    k_union_tiles<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     ++launches;
     k_compress<<<g, 256, 0, st>>>(a);
     ++launches;
-    k_border_tiles<<<(unsigned)a.nTiles, 128, 0, st>>>(a);
+    k_border_tiles<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     ++launches;
     k_root_flags<<<(a.n + 1 + 255) / 256, 256, 0, st>>>(a);
     ++launches;

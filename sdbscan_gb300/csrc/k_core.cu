@@ -93,16 +93,16 @@ __global__ void k_slot_sigs(const int32_t* __restrict__ topM, int D, int m, cons
     sig[q] = make_int4(o[0], o[1], o[2], c);
 }
 
-// multi[l][w] bit j: the point in slot 64 w + j of list l is held by another
+// multi[l][w] bit j: the point in slot CT w + j of list l is held by another
 // list too.  Most slots hold a point of one list only (about 84 % of the
 // passing pairs at 1M x 784); such an occurrence is the first and only one.
-__global__ void k_multi_bits(const int4* __restrict__ sig, int D, int m, int W, uint64_t* __restrict__ multi) {
+__global__ void k_multi_bits(const int4* __restrict__ sig, int D, int m, int W, int CT, uint64_t* __restrict__ multi) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= 2 * D * W) return;
     const int l = q / W, wd = q % W;
     uint64_t bits = 0;
-    for (int j = 0; j < 64 && wd * 64 + j < m; ++j)
-        bits |= (uint64_t)(sig[(size_t)l * m + wd * 64 + j].w > 0) << j;
+    for (int j = 0; j < CT && wd * CT + j < m; ++j)
+        bits |= (uint64_t)(sig[(size_t)l * m + wd * CT + j].w > 0) << j;
     multi[q] = bits;
 }
 
@@ -175,7 +175,7 @@ __device__ __forceinline__ void visit_point(const CoreArgs& a, uint32_t* km, con
                 for (int half = 0; half < 2; ++half) {
                     const int bit = half * 32 + (int)lane;
                     if ((mk >> bit) & 1ull) {
-                        const int s = wd * 64 + bit;
+                        const int s = wd * a.CT + bit;
                         const int i = __ldg(lst + s);
                         int mult;
                         bool isFirst;
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256, 4) k_core_dedupe(CoreArgs a, const int4* 
                 const int it = sw.item[t];
                 const int wl = it >> 6, bit = it & 63;
                 const int gg = wb + wl;
-                const int jj = gg / a.W, s = (gg % a.W) * 64 + bit;
+                const int jj = gg / a.W, s = (gg % a.W) * a.CT + bit;
                 const int l = sw.list[jj];
                 const int i = __ldg(a.topM + sw.rowOff[jj] + s);
                 int mult;
@@ -434,11 +434,11 @@ static int core_grid(int n, int warps) {
 }
 
 int launch_slot_sigs(const int32_t* topM, int D, int m, const int64_t* hubOff, const int32_t* hubLists, void* sig,
-                     uint64_t* multi, int W, cudaStream_t st) {
+                     uint64_t* multi, int W, int CT, cudaStream_t st) {
     const int total = 2 * D * m;
     k_slot_sigs<<<(total + 255) / 256, 256, 0, st>>>(topM, D, m, hubOff, hubLists, static_cast<int4*>(sig));
     if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    k_multi_bits<<<(2 * D * W + 255) / 256, 256, 0, st>>>(static_cast<const int4*>(sig), D, m, W, multi);
+    k_multi_bits<<<(2 * D * W + 255) / 256, 256, 0, st>>>(static_cast<const int4*>(sig), D, m, W, CT, multi);
     return cudaPeekAtLastError() == cudaSuccess ? 2 : -1;
 }
 

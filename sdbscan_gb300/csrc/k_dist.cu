@@ -146,14 +146,15 @@ template <int DIST, int TX, int CN, int KT = TK, int NST = STAGES> int launch_di
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
-// Tile shape: the caller's (autotuned) choice, else exact 50-column tiles for
-// m in 41..50 and 64-column tiles otherwise.  Variants: 1 = 128 x 64 (256
-// threads, 32 dimensions per stage, 2 stages), 2 = 128 x 50 (160 threads, 32
-// dimensions, 2 stages), 3 = 128 x 50 (160 threads, 16 dimensions, 4 stages:
-// the same shared memory, half the work between barriers and twice the loads
-// in flight; 3 % faster than 2 for Cosine at 1M x 784, 2.5 % slower for Chi2
-// at 500K x 512, so the other distances run shape 2 for it).  The 50-column
-// shapes need m <= 50.
+// Shape of the scalar tile: the caller's choice, else exact 50-column tiles
+// for m in 41..50 and 64-column tiles otherwise.  1 = 128 x 64 (256 threads,
+// 32 dimensions per stage, 2 stages), 2 = 128 x 50 (160 threads, the same
+// stages).  Where the packed tile (3, k_dist_pair.cu) is asked for but not
+// available -- Chi2 and JS, the BF16 screening's fallback, a candidate copy
+// that does not fit -- Cosine runs 128 x 50 with 16 dimensions in 4 stages
+// (the same shared memory, half the work between barriers and twice the loads
+// in flight; 3 % faster than 2 at 1M x 784, Chi2 2.5 % slower at 500K x 512).
+// The 50-column shapes need m <= 50.
 template <int DIST> int launch_dist_t(const DistArgs& a, cudaStream_t st) {
     const bool fits50 = a.m <= 50;
     if (a.variant == 4 || a.variant == 5) return launch_dist_ws(a, a.variant, st);
@@ -176,22 +177,22 @@ template <int DIST> int launch_dist_t(const DistArgs& a, cudaStream_t st) {
 // pattern of the reference's test_sDbscan, src/sDbscan.cpp:1009-1038).
 // Same tiles as k_dist; one warp per member row, lanes over candidates.
 __global__ void k_masks_from_dists(DistArgs a) {
-    __shared__ int colCount[TN];
+    __shared__ int colCount[64];
     __shared__ int passTotal;
     if ((int64_t)blockIdx.x >= *a.tileTotal) return;
     const int64_t t = tile_at(a.tilePerm, blockIdx.x);
     const int l = a.tileList[t];
     const int64_t ti = t - a.tileOff[l];
     const int mt = (int)(ti / a.nct), ct = (int)(ti % a.nct);
-    const int64_t mbeg = a.listOff[l] + (int64_t)mt * TM, mend = a.listOff[l + 1];
+    const int64_t mbeg = a.listOff[l] + (int64_t)mt * a.TM, mend = a.listOff[l + 1];
     const int r = l % a.nproj, side = l / a.nproj;
     const int32_t* cand = a.topM + (size_t)r * 2 * a.m + side * a.m;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int j = threadIdx.x; j < TN; j += blockDim.x) colCount[j] = 0;
+    for (int j = threadIdx.x; j < 64; j += blockDim.x) colCount[j] = 0;
     if (threadIdx.x == 0) passTotal = 0;
     __syncthreads();
     int myPass = 0;
-    for (int row = warp; row < TM; row += warps) {
+    for (int row = warp; row < a.TM; row += warps) {
         const int64_t q = mbeg + row;
         if (q >= mend) break;
         const int2 mb = a.members[q];
@@ -200,9 +201,9 @@ __global__ void k_masks_from_dists(DistArgs a) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int col = h * 32 + lane;
-            const int c = ct * TN + col;
+            const int c = ct * a.CT + col;
             bool pass = false;
-            if (c < a.m) {
+            if (col < a.CT && c < a.m) {
                 const int cp = __ldg(cand + c);
                 const size_t at = ((size_t)p * 2 * a.k + slot) * a.m + c;
                 const float dd = __ldg(a.dists + at);
@@ -219,8 +220,8 @@ __global__ void k_masks_from_dists(DistArgs a) {
     const int wp = warp_sum(myPass);
     if (lane == 0 && wp) atomicAdd(&passTotal, wp);
     __syncthreads();
-    for (int j = threadIdx.x; j < TN; j += blockDim.x) {
-        const int c = ct * TN + j;
+    for (int j = threadIdx.x; j < a.CT; j += blockDim.x) {
+        const int c = ct * a.CT + j;
         if (colCount[j]) atomicAdd(a.inRaw + cand[c], colCount[j]);
     }
     if (threadIdx.x == 0 && passTotal) atomicAdd(a.pairs, (unsigned long long)passTotal);
@@ -237,15 +238,15 @@ __global__ void k_pair_rounds(const float* __restrict__ dists, DistArgs a, uint3
     const size_t count = (size_t)a.n * 2 * a.k * g4;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / g4;
-        const int c0 = (int)(i % g4) * 4;
+        const int w0 = (int)(i % g4) * 4, c0 = w0 / 64 * a.CT, b0 = w0 % 64;  // word's first column, byte in the word
         const int p = (int)(row / (2 * a.k)), slot = (int)(row % (2 * a.k));
         const int32_t* cand = a.topM + (size_t)__ldg(a.topKmat + row) * 2 * a.m + (slot >= a.k ? a.m : 0);
         uint32_t out = 0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int c = c0 + b;
+            const int c = c0 + b0 + b;
             int r = 255;
-            if (c < a.m && __ldg(cand + c) != p) {
+            if (b0 + b < a.CT && c < a.m && __ldg(cand + c) != p) {
                 const float d = __ldg(dists + row * a.m + c);
                 r = 0;
                 while (r < a.nSweep && a.sweepEps[r] < d) ++r;
@@ -260,17 +261,17 @@ __global__ void k_pair_rounds(const float* __restrict__ dists, DistArgs a, uint3
 // row's 64 round bytes for this tile come in as four 16-byte loads and are
 // compared four at a time (__vcmpeq4), giving the row's mask word directly;
 // the column counts (reverse edges) are reduced with one ballot per column.
-__global__ void __launch_bounds__(TM) k_masks_from_rounds(DistArgs a) {
-    __shared__ int colCount[TN];
+__global__ void __launch_bounds__(256) k_masks_from_rounds(DistArgs a) {
+    __shared__ int colCount[64];
     if ((int64_t)blockIdx.x >= *a.tileTotal) return;
     const int64_t t = tile_at(a.tilePerm, blockIdx.x);
     const int l = a.tileList[t];
     const int64_t ti = t - a.tileOff[l];
     const int mt = (int)(ti / a.nct), ct = (int)(ti % a.nct);
-    const int64_t q = a.listOff[l] + (int64_t)mt * TM + threadIdx.x;
+    const int64_t q = a.listOff[l] + (int64_t)mt * a.TM + threadIdx.x;
     const bool valid = q < a.listOff[l + 1];
     const int lane = threadIdx.x & 31;
-    if (threadIdx.x < TN) colCount[threadIdx.x] = 0;
+    if (threadIdx.x < 64) colCount[threadIdx.x] = 0;
     __syncthreads();
     uint64_t w = 0;
     int2 mb = make_int2(0, 0);
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(TM) k_masks_from_rounds(DistArgs a) {
     }
     int cc0 = 0, cc1 = 0;  // passes of columns lane and lane + 32 in this warp
 #pragma unroll
-    for (int col = 0; col < TN; ++col) {
+    for (int col = 0; col < 64; ++col) {
         const int pc = __popc(__ballot_sync(0xffffffffu, (w >> col) & 1ull));
         if (lane == (col & 31)) {
             if (col < 32) cc0 += pc;
@@ -306,9 +307,9 @@ __global__ void __launch_bounds__(TM) k_masks_from_rounds(DistArgs a) {
     const int wp = warp_sum(__popcll(w));
     if (lane == 0 && wp) atomicAdd(a.pairs, (unsigned long long)wp);
     __syncthreads();
-    if (threadIdx.x < TN && colCount[threadIdx.x]) {
+    if (threadIdx.x < 64 && colCount[threadIdx.x]) {
         const int r = l % a.nproj, side = l / a.nproj;
-        const int c = ct * TN + threadIdx.x;
+        const int c = ct * a.CT + threadIdx.x;
         atomicAdd(a.inRaw + __ldg(a.topM + (size_t)r * 2 * a.m + side * a.m + c), colCount[threadIdx.x]);
     }
 }
@@ -322,7 +323,7 @@ int launch_pair_rounds(const DistArgs& a, uint8_t* rounds, cudaStream_t st) {
 
 int launch_masks_from_dists(const DistArgs& a, cudaStream_t st) {
     if (a.nTiles <= 0) return 0;
-    if (a.pairRound != nullptr) k_masks_from_rounds<<<(unsigned)a.nTiles, TM, 0, st>>>(a);
+    if (a.pairRound != nullptr) k_masks_from_rounds<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     else k_masks_from_dists<<<(unsigned)a.nTiles, 256, 0, st>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
