@@ -47,29 +47,69 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
     return true;
 }
 
+// Before the tile pass: rounds of hooking without unites.  A core point (in an
+// eps sweep one that became core this round) looks at two passing candidates
+// of two of its lists and hooks its root under the smallest root it sees, by a
+// plain atomicMin: parents only move down, so the forest stays a forest, and
+// where one root is hooked twice the tile pass, which sees every edge, restores
+// the other link.  With every point a set of its own the tile pass would send
+// some twenty unites per point at the same few roots, all at once; after the
+// rounds it finds mostly equal roots (50K x 128: union 379 us without, 100 plus
+// 45 for the rounds; 1M x 784: 1827 and 955 + 292).
+__global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.n || !a.core[p] || (a.carry && a.coreEps[p] != a.round)) return;
+    const int r = load_parent(a.parent, p);
+    int best = r;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int j = (slot0 + t) % (2 * a.k);
+        const size_t at = (size_t)p * 2 * a.k + j;
+        uint64_t bits = __ldg(reinterpret_cast<const unsigned long long*>(a.masks) + at * a.W);
+        if (!bits) continue;
+        const int32_t* cand = a.topM + (size_t)__ldg(a.topK + at) * 2 * a.m + (j >= a.k ? a.m : 0);
+        for (int c = 0; c < 2 && bits; ++c, bits &= bits - 1) {
+            const int q = __ldg(cand + __ffsll((long long)bits) - 1);
+            if (a.core[q]) best = min(best, load_parent(a.parent, q));
+        }
+    }
+    if (best < r) atomicMin(a.parent + r, best);
+}
+
+// The tile's candidates of one root, as a bit set.
+struct RootGroup {
+    unsigned long long bits;
+    int root;
+};
+
 // Union over the core-core edges of one tile.  The roots of the tile's core
-// candidates are found once and cached in shared memory; a member row then
-// compares its own root with the cached roots of its passing candidates and
-// unites only where they differ.  A cached value is always an ancestor of its
-// candidate (parents only move up), so equality proves the same set; a stale
-// value only costs a redundant unite.
+// candidates are found once and the candidates grouped by root in shared
+// memory; a member row then takes one step per group instead of one per
+// passing candidate: it unites where the group's root differs from its own.
+// A cached root is always an ancestor of its candidates (parents only move
+// up), so equality proves the same set; a stale one only costs a redundant
+// unite.
 __global__ void __launch_bounds__(256) k_union_tiles(ClusterArgs a) {
-    __shared__ int croot[64];
+    __shared__ RootGroup group[64];
+    __shared__ int groups;
     __shared__ unsigned long long newCoreCand;  // carry: candidates that became core this round
     Tile tl;
     if (!tile_of(a, blockIdx.x, tl)) return;
-    volatile int* vroot = croot;
-    if (threadIdx.x == 0) newCoreCand = 0ull;
+    if (threadIdx.x == 0) {
+        newCoreCand = 0ull;
+        groups = 0;
+    }
     __syncthreads();
-    int q = -1;  // this thread's candidate (threads < 64)
+    int q = -1;  // this thread's core candidate (threads < 64)
     if (threadIdx.x < 64) {
         const int c = tl.ct * a.CT + threadIdx.x;
         if ((int)threadIdx.x < a.CT && c < a.m) {
             q = __ldg(tl.cand + c);
-            if (a.carry && a.core[q] && a.coreEps[q] == a.round) atomicOr(&newCoreCand, 1ull << threadIdx.x);
+            if (!a.core[q]) q = -1;
+            else if (a.carry && a.coreEps[q] == a.round) atomicOr(&newCoreCand, 1ull << threadIdx.x);
         }
     }
-    __syncthreads();
+    if (a.carry) __syncthreads();
     const int64_t row = tl.mbeg + threadIdx.x;
     int p = -1;
     uint64_t bits = 0;
@@ -86,18 +126,25 @@ __global__ void __launch_bounds__(256) k_union_tiles(ClusterArgs a) {
         }
     }
     if (!__syncthreads_or(bits != 0)) return;  // nothing to unite in this tile
-    if (threadIdx.x < 64) croot[threadIdx.x] = (q >= 0 && a.core[q]) ? find_root(a.parent, q) : -1;
+    if (threadIdx.x < 64) {
+        const int root = q >= 0 ? find_root(a.parent, q) : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, root);
+        if (root >= 0 && (int)lane_id() == __ffs((int)same) - 1) {
+            RootGroup& g = group[atomicAdd(&groups, 1)];
+            g.bits = (unsigned long long)same << (threadIdx.x & 32);
+            g.root = root;
+        }
+    }
     __syncthreads();
     if (!bits) return;
     int rp = find_root(a.parent, p);
-    while (bits) {
-        const int j = __ffsll((long long)bits) - 1;
-        bits &= bits - 1;
-        const int cr = vroot[j];
-        if (cr < 0 || cr == rp) continue;
+    const int ng = groups;
+    for (int g = 0; g < ng; ++g) {
+        const int cr = reinterpret_cast<volatile int&>(group[g].root);
+        if (cr == rp || !(bits & group[g].bits)) continue;
         unite(a.parent, rp, cr);
         rp = find_root(a.parent, rp);
-        vroot[j] = rp;
+        reinterpret_cast<volatile int&>(group[g].root) = rp;
     }
 }
 
@@ -110,46 +157,50 @@ __global__ void k_compress(ClusterArgs a) {
 // Border labels of one tile (parents are roots after k_compress).  A non-core
 // member takes the smallest root among its passing core candidates; a non-core
 // candidate takes the smallest root among the core members passing with it,
-// reduced in shared memory first so each candidate sees one global atomic.
+// reduced in shared memory first so each candidate sees one global atomic.  A
+// core member's mask word is read only where the tile has a non-core candidate
+// (1M x 784, every point core: 772 -> 181 us).
 __global__ void __launch_bounds__(256) k_border_tiles(ClusterArgs a) {
-    __shared__ int croot[64], cbest[64], cpt[64];
+    __shared__ int croot[64], cbest[64];
+    __shared__ unsigned nonCore[2];  // the tile's non-core candidates
     Tile tl;
     if (!tile_of(a, blockIdx.x, tl)) return;
+    int q = -1;
     if (threadIdx.x < 64) {
         const int c = tl.ct * a.CT + threadIdx.x;
-        const int q = (int)threadIdx.x < a.CT && c < a.m ? __ldg(tl.cand + c) : -1;
-        cpt[threadIdx.x] = q;
-        croot[threadIdx.x] = (q >= 0 && a.core[q]) ? __ldcg(a.parent + q) : INT_MAX;
+        q = (int)threadIdx.x < a.CT && c < a.m ? __ldg(tl.cand + c) : -1;
+        const bool core = q >= 0 && a.core[q];
+        croot[threadIdx.x] = core ? __ldcg(a.parent + q) : INT_MAX;
         cbest[threadIdx.x] = INT_MAX;
+        const unsigned b = __ballot_sync(0xffffffffu, q >= 0 && !core);
+        if (lane_id() == 0) nonCore[threadIdx.x >> 5] = b;
     }
     __syncthreads();
+    const uint64_t nc = ((uint64_t)nonCore[1] << 32) | nonCore[0];
     const int64_t row = tl.mbeg + threadIdx.x;
     if (row < tl.mend) {
         const int2 mb = __ldg(a.members + row);
         const int p = mb.x;
-        uint64_t bits = __ldg(reinterpret_cast<const unsigned long long*>(a.masks) +
-                              ((size_t)p * 2 * a.k + mb.y) * a.W + tl.ct);
-        if (bits) {
-            if (a.core[p]) {
+        const bool core = a.core[p];
+        uint64_t bits = 0;
+        if (!core || nc)
+            bits = __ldg(reinterpret_cast<const unsigned long long*>(a.masks) + ((size_t)p * 2 * a.k + mb.y) * a.W +
+                         tl.ct);
+        if (core) {
+            bits &= nc;
+            if (bits) {
                 const int rp = __ldcg(a.parent + p);
-                while (bits) {
-                    const int j = __ffsll((long long)bits) - 1;
-                    bits &= bits - 1;
-                    if (croot[j] == INT_MAX) atomicMin(&cbest[j], rp);
-                }
-            } else {
-                int best = INT_MAX;
-                while (bits) {
-                    const int j = __ffsll((long long)bits) - 1;
-                    bits &= bits - 1;
-                    best = min(best, croot[j]);
-                }
-                if (best != INT_MAX) atomicMin(a.border + p, best);
+                for (; bits; bits &= bits - 1) atomicMin(&cbest[__ffsll((long long)bits) - 1], rp);
             }
+        } else {
+            int best = INT_MAX;
+            for (; bits; bits &= bits - 1) best = min(best, croot[__ffsll((long long)bits) - 1]);
+            if (best != INT_MAX) atomicMin(a.border + p, best);
         }
     }
+    if (!nc) return;
     __syncthreads();
-    if (threadIdx.x < 64 && cbest[threadIdx.x] != INT_MAX) atomicMin(a.border + cpt[threadIdx.x], cbest[threadIdx.x]);
+    if (q >= 0 && cbest[threadIdx.x] != INT_MAX) atomicMin(a.border + q, cbest[threadIdx.x]);
 }
 
 __global__ void k_root_flags(ClusterArgs a) {
@@ -178,6 +229,15 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st) {
     const int g = (a.n + 255) / 256;
     k_init<<<g, 256, 0, st>>>(a.parent, a.border, a.n, a.carry && a.round > 0);
     ++launches;
+    // three rounds over two lists, two candidates of each (33K x 333 cluster
+    // stage: 0.49 ms with one round over one candidate, 0.35 with two rounds,
+    // 0.26 with three); a sweep's later rounds have few new core points
+    const int rounds = !a.carry ? 3 : a.round == 0 ? 2 : 1;
+    for (int t = 0; t < rounds; ++t) {
+        k_hook<<<g, 256, 0, st>>>(a, 2 * t);
+        k_compress<<<g, 256, 0, st>>>(a);
+        launches += 2;
+    }
     k_union_tiles<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     ++launches;
     k_compress<<<g, 256, 0, st>>>(a);
