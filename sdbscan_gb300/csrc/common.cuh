@@ -281,15 +281,23 @@ struct CoreArgs {
     int accumulate, round;
     uint64_t* newMasks;      // n x 2k x W (accumulate only)
     int32_t* coreEps;        // n: round at which the point became core, -1 before (accumulate only)
-    const uint64_t* multi;   // 2D x W: slots whose point another list holds too (launch_slot_sigs)
+    // points that two or more lists hold (launch_hub_index)
+    const uint64_t* multi;      // 2D x W: the slots that hold one
+    const int32_t* slotMulti;   // D x 2m: its dense number, -1 for the other slots
+    const int32_t* slotHub;     // D x 2m: hubIdx of the slot's point
+    const unsigned long long* multiCount;  // device: how many there are
 };
-// Per-slot signatures (sig, 2D x m int4) and the multi-list slot bits (multi, 2D x W).
+// sOPTICS: per-slot signatures (sig, 2D x m int4).
 int launch_slot_sigs(const int32_t* topM, int D, int m, const int64_t* hubOff, const int32_t* hubLists, void* sig,
-                     uint64_t* multi, int W, int CT, cudaStream_t st);
-int launch_core_dedupe(const CoreArgs& a, const void* sig, cudaStream_t st);
-// hubIdx from hubOff (a scan of hub flags into idxTmp) and the hubs' list masks.
-int launch_hub_masks(const CoreArgs& a, int32_t* hubIdx, int64_t* idxTmp, uint32_t* kMask, int64_t* scanTmp,
-                     int64_t* nHubsDev, cudaStream_t st);
+                     cudaStream_t st);
+int launch_core_dedupe(const CoreArgs& a, cudaStream_t st);
+// From hubOff: dense hub numbers (hubIdx, n; hubPoint, its inverse) and the
+// hubs' list masks, dense numbers of the points of two or more lists (multiIdx,
+// n) and what CoreArgs keeps of them; count[0], count[1] (zeroed by the caller)
+// receive how many there are.
+int launch_hub_index(const CoreArgs& a, int32_t* hubIdx, int32_t* hubPoint, int32_t* multiIdx, uint32_t* kMask,
+                     int32_t* slotMulti, int32_t* slotHub, uint64_t* multi, unsigned long long* count,
+                     cudaStream_t st);
 int launch_core_finish(const CoreArgs& a, cudaStream_t st);
 
 struct ClusterArgs {

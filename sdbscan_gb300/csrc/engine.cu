@@ -128,7 +128,8 @@ std::vector<DevBuf*> sdb_engine::all_bufs() {
             &kMask, &firstMasks, &Xb, &queue, &sweepLabels, &sweepNcl, &sig, &Rb, &newMasks, &coreEps, &sampleFlag,
             &noiseFlag, &noiseCores, &noisePts, &PcT, &numCore, &pairRound, &sngCols, &sngMult, &sngColOf, &sngExtras,
             &sngExtraPass, &sngMask, &rowDeg, &colCnt, &sngUb, &sngHeavy, &chunkOff, &tileKey, &keyOff, &tilePerm,
-            &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask};
+            &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask,
+            &multiIdx, &slotMulti, &slotHub, &hubPoint};
 }
 
 // ---------------------------------------------------------------------------
@@ -300,7 +301,10 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     const int maskWords = (L + 31) / 32;
     const size_t maxHubs = std::min<size_t>((size_t)n, (size_t)L * m);
     ok &= ensure(hubIdx, sizeof(int32_t) * n) && ensure(kMask, sizeof(uint32_t) * maxHubs * maskWords) &&
-          ensure(sig, 16 * (size_t)L * m) && ensure(multiMask, sizeof(uint64_t) * (size_t)L * W);
+          ensure(multiMask, sizeof(uint64_t) * (size_t)L * W) && ensure(multiIdx, sizeof(int32_t) * n) &&
+          ensure(hubPoint, sizeof(int32_t) * maxHubs) &&
+          ensure(slotMulti, sizeof(int32_t) * (size_t)L * m) && ensure(slotHub, sizeof(int32_t) * (size_t)L * m);
+    if (optics) ok &= ensure(sig, 16 * (size_t)L * m);
     if (rff) ok &= ensure(E, sizeof(float) * (size_t)n * ker) && ensure(Rt, sizeof(float) * hostRt.size());
     if (optics || sweep) ok &= ensure(dists, sizeof(float) * (size_t)n * 2 * k * m);
     if (optics) ok &= ensure(coreDist, sizeof(float) * n);
@@ -487,8 +491,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     L_(launch_scan_i64(i64(hubOff), i64(hubOff), (size_t)n + 1, i64(scanTmp), st));
     SDB_CK(cudaMemsetAsync(hubCount.ptr, 0, sizeof(int32_t) * n, st));
     L_(launch_hubs_scatter(ia, st));
-    L_(launch_slot_sigs(i32(topM), D, m, i64(hubOff), i32(hubLists), sig.ptr, static_cast<uint64_t*>(multiMask.ptr), W,
-                        CT, st));
+    if (optics) L_(launch_slot_sigs(i32(topM), D, m, i64(hubOff), i32(hubLists), sig.ptr, st));
     if (!ok) return fail(SDB_ERR_CUDA, std::string("index launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     if (!capture) SDB_CK(cudaEventRecord(ev[4], st));
 
@@ -590,6 +593,9 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     ca.hubOff = i64(hubOff);
     ca.hubLists = i32(hubLists);
     ca.multi = static_cast<const uint64_t*>(multiMask.ptr);
+    ca.slotMulti = i32(slotMulti);
+    ca.slotHub = i32(slotHub);
+    ca.multiCount = ctr + 6;
     ca.inRaw = i32(inRaw);
     ca.aCount = i32(aCount);
     ca.degree = i32(degree);
@@ -599,9 +605,8 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     ca.hubIdx = i32(hubIdx);
     ca.kMask = static_cast<const uint32_t*>(kMask.ptr);
     ca.firstMasks = static_cast<uint64_t*>(firstMasks.ptr);
-    SDB_CK(cudaMemsetAsync(kMask.ptr, 0, sizeof(uint32_t) * maxHubs * maskWords, st));
-    L_(launch_hub_masks(ca, i32(hubIdx), i64(rootFlag), static_cast<uint32_t*>(kMask.ptr), i64(scanTmp),
-                        reinterpret_cast<int64_t*>(ctr + 5), st));
+    L_(launch_hub_index(ca, i32(hubIdx), i32(hubPoint), i32(multiIdx), static_cast<uint32_t*>(kMask.ptr),
+                        i32(slotMulti), i32(slotHub), static_cast<uint64_t*>(multiMask.ptr), ctr + 5, st));
     const int rounds = sweep ? sw->nEps : 1;
     // an eps sweep runs in ascending eps: each round adds the pairs with
     // previous eps < d <= eps to the degrees, the first-occurrence masks and
@@ -637,7 +642,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
         SDB_CK(cudaMemsetAsync(inRaw.ptr, 0, sizeof(int32_t) * n, st));
         L_(launch_masks_from_dists(da, st));
     }
-    L_(launch_core_dedupe(ca, sig.ptr, st));
+    L_(launch_core_dedupe(ca, st));
     L_(launch_core_finish(ca, st));
     if (!ok) return fail(SDB_ERR_CUDA, std::string("core launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     if (!capture) SDB_CK(cudaEventRecord(ev[6], st));

@@ -22,6 +22,27 @@
 namespace sdb {
 namespace {
 
+// true iff one of the lists point i meets through its top-k is in listMask:
+// i's entries two at a time, four loads in flight (2k is even and a row starts
+// on 8 bytes).
+__device__ __forceinline__ bool meets_list(const CoreArgs& a, const uint32_t* listMask, int i) {
+    const int2* ki = reinterpret_cast<const int2*>(a.topK + (size_t)i * 2 * a.k);
+    for (int j = 0; j < a.k; j += 4) {
+        int2 e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u] = __ldg(ki + min(j + u, a.k - 1));
+        uint32_t hit = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int j2 = 2 * min(j + u, a.k - 1);
+            const int l0 = e[u].x + (j2 >= a.k ? a.nproj : 0), l1 = e[u].y + (j2 + 1 >= a.k ? a.nproj : 0);
+            hit |= (listMask[l0 >> 5] >> (l0 & 31)) | (listMask[l1 >> 5] >> (l1 & 31));
+        }
+        if (hit & 1u) return true;
+    }
+    return false;
+}
+
 // true iff hub point p is in one of point i's 2k candidate lists, i.e. one
 // of the top-m lists holding p is among the lists i meets through its top-k.
 // Two equivalent tests; the cheaper one for p is used:
@@ -39,37 +60,82 @@ __device__ __forceinline__ bool in_candidates_of(const CoreArgs& a, const uint32
         }
         return false;
     }
-    const int32_t* ki = a.topK + (size_t)i * 2 * a.k;
-    for (int j = 0; j < 2 * a.k; ++j) {
-        const int lst = __ldg(ki + j) + (j >= a.k ? a.nproj : 0);
-        if ((listMask[lst >> 5] >> (lst & 31)) & 1u) return true;
+    return meets_list(a, listMask, i);
+}
+
+// Dense numbers (any order: they only name rows and bits) for the hubs and for
+// the points that two or more lists hold.
+__global__ void __launch_bounds__(256) k_hub_index(CoreArgs a, int32_t* __restrict__ hubIdx,
+                                                   int32_t* __restrict__ hubPoint, int32_t* __restrict__ multiIdx,
+                                                   unsigned long long* __restrict__ count) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lane = lane_id();
+    const int lists = p < a.n ? (int)(a.hubOff[p + 1] - a.hubOff[p]) : 0;
+    const unsigned hubs = __ballot_sync(0xffffffffu, lists > 0), multi = __ballot_sync(0xffffffffu, lists > 1);
+    unsigned long long base = 0;
+    if (lane < 2) {
+        const int c = __popc(lane ? multi : hubs);
+        if (c) base = atomicAdd(count + lane, (unsigned long long)c);
     }
-    return false;
-}
-
-__global__ void k_hub_flags(const int64_t* __restrict__ hubOff, int n, int64_t* __restrict__ flag) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p <= n) flag[p] = (p < n && hubOff[p + 1] > hubOff[p]) ? 1 : 0;
-}
-
-__global__ void k_hub_index(CoreArgs a, const int64_t* __restrict__ scanned, int32_t* __restrict__ hubIdx,
-                            uint32_t* __restrict__ kMask, int64_t* __restrict__ nHubs) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) *nHubs = scanned[a.n];
+    const unsigned below = (1u << lane) - 1u;
+    const int h = (int)__shfl_sync(0xffffffffu, base, 0) + __popc(hubs & below);
+    const int u = (int)__shfl_sync(0xffffffffu, base, 1) + __popc(multi & below);
     if (p >= a.n) return;
-    const bool hub = a.hubOff[p + 1] > a.hubOff[p];
-    const int h = hub ? (int)scanned[p] : -1;
-    hubIdx[p] = h;
-    if (!hub) return;
-    const int words = (2 * a.nproj + 31) / 32;
-    uint32_t* km = kMask + (size_t)h * words;
-    for (int j = 0; j < 2 * a.k; ++j) {
-        const int lst = a.topK[(size_t)p * 2 * a.k + j] + (j >= a.k ? a.nproj : 0);
-        atomicOr(km + (lst >> 5), 1u << (lst & 31));
+    hubIdx[p] = lists > 0 ? h : -1;
+    multiIdx[p] = lists > 1 ? u : -1;
+    if (lists > 0) hubPoint[h] = p;
+}
+
+// The hubs' list masks, a warp per hub, a word per lane.
+__global__ void __launch_bounds__(256) k_hub_masks(CoreArgs a, const int32_t* __restrict__ hubPoint,
+                                                   const unsigned long long* __restrict__ count,
+                                                   uint32_t* __restrict__ kMask) {
+    const int h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (h >= (int)__ldg(count)) return;
+    const int lane = (int)lane_id(), words = (2 * a.nproj + 31) / 32, slots = 2 * a.k;
+    const int32_t* tk = a.topK + (size_t)__ldg(hubPoint + h) * slots;
+    const int lA = lane < slots ? __ldg(tk + lane) + (lane >= a.k ? a.nproj : 0) : 0;
+    const int lB = lane + 32 < slots ? __ldg(tk + lane + 32) + (lane + 32 >= a.k ? a.nproj : 0) : 0;
+    for (int w0 = 0; w0 < words; w0 += 32) {
+        uint32_t bits = 0;
+        for (int j = 0; j < slots; ++j) {
+            const int l = __shfl_sync(0xffffffffu, j < 32 ? lA : lB, j & 31);
+            if (l >> 5 == w0 + lane) bits |= 1u << (l & 31);
+        }
+        if (w0 + lane < words) kMask[(size_t)h * words + w0 + lane] = bits;
     }
 }
 
-// Duplicates without hashing.  Point p meets candidate i once per list of p
+// A warp per (list, word): slotMulti and slotHub = multiIdx and hubIdx of the
+// slot's point, in topM's layout, and multi[l][w] bit j: the point in slot CT w + j of list l is held
+// by another list too.  Most slots hold a point of one list only (about 84 % of
+// the passing pairs at 1M x 784); such an occurrence is the first and only one.
+__global__ void __launch_bounds__(256) k_slot_multi(const int32_t* __restrict__ topM, int D, int m, int W, int CT,
+                                                    const int32_t* __restrict__ multiIdx,
+                                                    const int32_t* __restrict__ hubIdx,
+                                                    int32_t* __restrict__ slotMulti, int32_t* __restrict__ slotHub,
+                                                    uint64_t* __restrict__ multi) {
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (q >= 2 * D * W) return;
+    const int l = q / W, wd = q % W;
+    const size_t row = (size_t)(l % D) * 2 * m + (l / D) * m;
+    uint32_t half[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = h * 32 + (int)lane_id(), s = wd * CT + c;
+        int u = -1;
+        if (c < CT && s < m) {
+            const int i = __ldg(topM + row + s);
+            u = __ldg(multiIdx + i);
+            slotMulti[row + s] = u;
+            slotHub[row + s] = __ldg(hubIdx + i);
+        }
+        half[h] = __ballot_sync(0xffffffffu, u >= 0);
+    }
+    if (lane_id() == 0) multi[q] = ((uint64_t)half[1] << 32) | half[0];
+}
+
+// The sOPTICS emission's first occurrences.  Point p meets candidate i once per list of p
 // that holds i, so with K(p) = p's 2k lists and L(i) = the top-m lists
 // holding i, i's multiplicity among p's candidates is |K(p) n L(i)|, and the
 // occurrence through list l is the first one iff no smaller list of
@@ -91,19 +157,6 @@ __global__ void k_slot_sigs(const int32_t* __restrict__ topM, int D, int m, cons
         ++c;
     }
     sig[q] = make_int4(o[0], o[1], o[2], c);
-}
-
-// multi[l][w] bit j: the point in slot CT w + j of list l is held by another
-// list too.  Most slots hold a point of one list only (about 84 % of the
-// passing pairs at 1M x 784); such an occurrence is the first and only one.
-__global__ void k_multi_bits(const int4* __restrict__ sig, int D, int m, int W, int CT, uint64_t* __restrict__ multi) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= 2 * D * W) return;
-    const int l = q / W, wd = q % W;
-    uint64_t bits = 0;
-    for (int j = 0; j < CT && wd * CT + j < m; ++j)
-        bits |= (uint64_t)(sig[(size_t)l * m + wd * CT + j].w > 0) << j;
-    multi[q] = bits;
 }
 
 __device__ __forceinline__ bool has_list(const uint32_t* km, int lst) { return (km[lst >> 5] >> (lst & 31)) & 1u; }
@@ -204,121 +257,164 @@ __device__ __forceinline__ void mark_lists(const CoreArgs& a, uint32_t* listMask
     __syncwarp();
 }
 
-// Per-warp shared memory of k_core_dedupe (after the two list masks).
-constexpr int kDdWords = 32;   // mask words per round, one per lane
-constexpr int kDdSlots = 62;   // 2k for k <= 31
-struct DedupeWarp {
-    uint32_t fresh[2 * kDdWords];       // first-occurrence bits found by the per-pair test (32-bit halves)
-    int32_t list[kDdSlots];             // per slot: its list
-    int32_t rowOff[kDdSlots];           // per slot: its list's row in topM
-    uint16_t item[kDdWords * 64];       // the round's pairs that need the per-pair test: (word, bit)
+// Per-warp shared memory of k_core_dedupe, between the seen bits and p's list mask.
+constexpr int kDdHalves = 32;      // mask half-words (32 bits) per round, one per lane
+constexpr int kDdLists = 8;        // lists of a hub tested against the candidates' list masks
+constexpr int kDdSeenWords = 1024; // seen bits held at once: 32768 points (more are taken in passes)
+struct alignas(16) DedupeWarp {
+    uint32_t drop[kDdHalves];      // gathered pairs that are no first occurrence
+    int32_t off[kDdHalves];        // the half-word's first slot in topM
+    uint16_t item[kDdHalves * 32]; // the round's pairs that need the per-pair test: (half-word, bit)
+    int32_t lists[kDdLists];       // a hub's lists, when it has at most that many
 };
-__host__ __device__ constexpr size_t dedupe_warp_bytes(int maskWords) {
-    return sizeof(uint32_t) * 2 * (size_t)maskWords + sizeof(DedupeWarp);
+__host__ __device__ constexpr size_t dedupe_warp_bytes(int seenWords, int maskWords) {
+    return (sizeof(uint32_t) * ((size_t)seenWords + maskWords) + sizeof(DedupeWarp) + 15) / 16 * 16;
 }
 
-// Persistent warps, each over points p = warp, warp + total, ...
-// A point that is no hub (no top-m list holds it) takes the pairs whose
-// candidate no other list holds straight from the mask words (first
-// occurrence, multiplicity 1, nothing to correct) and runs the per-pair test
-// only on the others; a hub runs it on all its pairs, since each of its first
-// occurrences needs the in-candidates test too.  The pairs to test are first
-// gathered into a dense per-warp list, so the warp's instructions follow those
-// pairs rather than every slot and lane.
-__global__ void __launch_bounds__(256, 4) k_core_dedupe(CoreArgs a, const int4* __restrict__ sig) {
-    extern __shared__ __align__(16) uint32_t shm[];
+// Persistent warps, each over points p = warp, warp + total, ...  A candidate
+// that no other list holds is a first occurrence as it stands.  The others are
+// gathered into a dense per-warp list (so the warp's instructions follow those
+// pairs, not every slot and lane) and set one bit each in a shared-memory bit
+// row indexed by multiIdx: the occurrence that finds the bit clear is the
+// first (which one it is does not matter to any later stage), every other one
+// takes itself out of the candidate's count.  A hub's first occurrences need
+// the in-candidates test, so all its pairs are gathered.
+// (Signatures per slot tested against the point's lists, the form before, walk
+// a candidate's lists where more than four hold it.  Core stage then and now:
+// 2K x 64, 51 lists a point, 317 -> 62 us; 50K x 128 328 -> 211; 1M x 784
+// 2147 -> 1744.)  Bound: L2 latency of the slot and list-mask loads, then
+// shared-memory wavefronts (61 % at 200K x 784).
+__global__ void __launch_bounds__(128, 8) k_core_dedupe(CoreArgs a, int seenWords) {
+    extern __shared__ __align__(16) unsigned char ddShm[];
     const int w = threadIdx.x >> 5;
-    const unsigned lane = lane_id();
+    const int lane = (int)lane_id();
     const int maskWords = (2 * a.nproj + 31) / 32;
-    uint32_t* km = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(shm) + (size_t)w * dedupe_warp_bytes(maskWords));
-    uint32_t* listMask = km + maskWords;
-    DedupeWarp& sw = *reinterpret_cast<DedupeWarp*>(listMask + maskWords);
-    for (int t = (int)lane; t < maskWords; t += 32) km[t] = 0u;
-    __syncwarp();
+    uint32_t* seen = reinterpret_cast<uint32_t*>(ddShm + (size_t)w * dedupe_warp_bytes(seenWords, maskWords));
+    DedupeWarp& sw = *reinterpret_cast<DedupeWarp*>(seen + seenWords);
+    uint32_t* listMask = reinterpret_cast<uint32_t*>(&sw + 1);
     const int gw = blockIdx.x * (blockDim.x >> 5) + w;
     const int nw = gridDim.x * (blockDim.x >> 5);
     const int slots = 2 * a.k;
-    const int nWords = slots * a.W;
-    const unsigned long long* mk64 = reinterpret_cast<const unsigned long long*>(a.masks);
+    const int nHalves = 2 * slots * a.W;
+    const uint32_t* mk32 = reinterpret_cast<const uint32_t*>(a.masks);
+    const uint32_t* mu32 = reinterpret_cast<const uint32_t*>(a.multi);
+    uint32_t* out = reinterpret_cast<uint32_t*>(a.accumulate ? a.newMasks : a.firstMasks);
+    uint32_t* all = reinterpret_cast<uint32_t*>(a.firstMasks);
+    const int multi = (int)__ldg(a.multiCount), span = seenWords * 32;
     for (int p = gw; p < a.n; p += nw) {
-        const unsigned long long* pm = mk64 + (size_t)p * nWords;
+        const size_t row = (size_t)p * nHalves;
         // a point without a passing pair (common in a sweep round) only clears
         // its first-occurrence words (this round's words when accumulating)
         bool any = false;
-        for (int t = (int)lane; t < nWords; t += 32) any |= __ldg(pm + t) != 0ull;
+        for (int t = lane; t < nHalves; t += 32) any |= __ldg(mk32 + row + t) != 0u;
         if (!__any_sync(0xffffffffu, any)) {
-            uint64_t* out = a.accumulate ? a.newMasks : a.firstMasks;
-            for (int t = (int)lane; t < nWords; t += 32) out[(size_t)p * nWords + t] = 0ull;
+            for (int t = lane; t < nHalves; t += 32) out[row + t] = 0u;
             if (lane == 0) a.aCount[p] = 0;
             continue;
         }
-        const int64_t h0 = a.hubOff[p], h1 = a.hubOff[p + 1];
-        const bool hub = h1 > h0;
-        if (hub) mark_lists(a, listMask, h0, h1, maskWords);
-        for (int j = (int)lane; j < slots; j += 32) {
-            const int l = __ldg(a.topK + (size_t)p * slots + j) + (j >= a.k ? a.nproj : 0);
-            sw.list[j] = l;
-            sw.rowOff[j] = (l % a.nproj) * 2 * a.m + (l / a.nproj) * a.m;
-            atomicOr(km + (l >> 5), 1u << (l & 31));
+        const int64_t h0 = a.hubOff[p];
+        const int np = (int)(a.hubOff[p + 1] - h0);
+        const bool hub = np > 0;
+        const bool few = np <= kDdLists;
+        if (few) {
+            if (lane < np) sw.lists[lane] = a.hubLists[h0 + lane];
+        } else {
+            mark_lists(a, listMask, h0, h0 + np, maskWords);
         }
-        __syncwarp();
         int distinct = 0;
-        for (int wb = 0; wb < nWords; wb += kDdWords) {
-            const int g = wb + (int)lane;  // this lane's mask word: slot g / W, word g % W
-            uint64_t mk = 0, mu = 0;
-            if (g < nWords) {
-                mk = __ldg(pm + g);
-                // a hub's every first occurrence needs the in-candidates test
-                mu = hub ? ~0ull : __ldg(a.multi + (size_t)sw.list[g / a.W] * a.W + g % a.W);
-            }
-            const uint64_t sole = mk & ~mu, todo = mk & mu;
-            distinct += __popcll(sole);
-            sw.fresh[2 * lane] = 0u;
-            sw.fresh[2 * lane + 1] = 0u;
-            // gather the pairs that need the test: lane-serial over its word's bits
-            const int cnt = __popcll(todo);
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += v;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            int at = incl - cnt;
-            for (uint64_t t = todo; t; t &= t - 1) sw.item[at++] = (uint16_t)((lane << 6) | (__ffsll((long long)t) - 1));
-            __syncwarp();
-            for (int t = (int)lane; t < total; t += 32) {
-                const int it = sw.item[t];
-                const int wl = it >> 6, bit = it & 63;
-                const int gg = wb + wl;
-                const int jj = gg / a.W, s = (gg % a.W) * a.CT + bit;
-                const int l = sw.list[jj];
-                const int i = __ldg(a.topM + sw.rowOff[jj] + s);
-                int mult;
-                bool first;
-                occurrence(a, km, sig, l, s, i, mult, first);
-                if (!first) continue;
-                ++distinct;
-                atomicOr(&sw.fresh[2 * wl + (bit >> 5)], 1u << (bit & 31));
-                int corr = mult - 1;
-                if (hub && in_candidates_of(a, listMask, a.hubLists + h0, (int)(h1 - h0), i)) corr += 1;
-                if (corr) atomicSub(a.inRaw + i, corr);
-            }
-            __syncwarp();
-            if (g < nWords) {
-                const size_t o = (size_t)p * nWords + g;
-                const uint64_t f64 = sole | ((uint64_t)sw.fresh[2 * lane + 1] << 32) | sw.fresh[2 * lane];
-                if (a.accumulate) {
-                    a.firstMasks[o] |= f64;
-                    a.newMasks[o] = f64;
-                } else {
-                    a.firstMasks[o] = f64;
+        // pass s0 takes the candidates numbered [s0, s0 + span); the first one
+        // takes those of a single list too
+        for (int s0 = 0; s0 == 0 || s0 < multi; s0 += span) {
+            for (int t = lane; 128 * t < min(span, multi - s0); t += 32)
+                reinterpret_cast<uint4*>(seen)[t] = make_uint4(0u, 0u, 0u, 0u);
+            for (int hb = 0; hb < nHalves; hb += kDdHalves) {
+                const int g = hb + lane;  // this lane's half-word: word g / 2 of slot g / 2W
+                uint32_t mk = 0, mu = 0;
+                if (g < nHalves) {
+                    mk = __ldg(mk32 + row + g);
+                    const int word = g >> 1;
+                    const int jj = a.W == 1 ? word : word / a.W, wd = word - jj * a.W;
+                    const int r = __ldg(a.topK + (size_t)p * slots + jj), side = jj >= a.k;
+                    sw.off[lane] = r * 2 * a.m + side * a.m + wd * a.CT + (g & 1) * 32;
+                    mu = hub && s0 == 0
+                             ? ~0u
+                             : __ldg(mu32 + 2 * ((size_t)(r + (side ? a.nproj : 0)) * a.W + wd) + (g & 1));
                 }
+                const uint32_t sole = s0 == 0 ? mk & ~mu : 0u, todo = mk & mu;
+                distinct += __popc(sole);
+                sw.drop[lane] = 0u;
+                // gather the pairs that need the test: lane-serial over its half-word's bits
+                const int cnt = __popc(todo);
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                uint16_t* at = sw.item + (incl - cnt);
+                for (uint32_t t = todo; t; t &= t - 1) *at++ = (uint16_t)((lane << 5) | (__ffs((int)t) - 1));
+                __syncwarp();
+                // two pairs per lane and step, their loads together: the loop
+                // waits for L2, not for instructions
+                for (int t = lane; t < total; t += 64) {
+                    int it[2], u[2], i[2], h[2];
+                    bool have[2], first[2], out1[2];  // out1: one to take out of the candidate's count
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        have[e] = first[e] = t + 32 * e < total;
+                        it[e] = sw.item[have[e] ? t + 32 * e : t];
+                        const int off = sw.off[it[e] >> 5] + (it[e] & 31);
+                        u[e] = __ldg(a.slotMulti + off);
+                        i[e] = __ldg(a.topM + off);
+                        h[e] = hub ? __ldg(a.slotHub + off) : 0;
+                        out1[e] = false;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int b = u[e] - s0;
+                        if (first[e] && u[e] >= 0) {
+                            if ((unsigned)b >= (unsigned)span) {
+                                first[e] = false;  // another pass's
+                            } else if ((atomicOr(seen + (b >> 5), 1u << (b & 31)) >> (b & 31)) & 1u) {
+                                first[e] = false;  // a repeat of a candidate already counted
+                                out1[e] = true;
+                            }
+                        }
+                        // (marking the others: neighbouring lanes' pairs share a
+                        // half-word, and most are first occurrences)
+                        if (first[e]) ++distinct;
+                        else if (have[e]) atomicOr(&sw.drop[it[e] >> 5], 1u << (it[e] & 31));
+                    }
+                    if (few) {  // p in A(i): one of p's lists is among those i meets
+                        const uint32_t* km0 = a.kMask + (size_t)h[0] * maskWords;
+                        const uint32_t* km1 = a.kMask + (size_t)h[1] * maskWords;
+                        for (int q = 0; q < np; ++q) {
+                            const int l = sw.lists[q];
+                            const uint32_t w0 = first[0] ? __ldg(km0 + (l >> 5)) : 0u;
+                            const uint32_t w1 = first[1] ? __ldg(km1 + (l >> 5)) : 0u;
+                            out1[0] |= (w0 >> (l & 31)) & 1u;
+                            out1[1] |= (w1 >> (l & 31)) & 1u;
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            if (first[e]) out1[e] = meets_list(a, listMask, i[e]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (out1[e]) atomicSub(a.inRaw + i[e], 1);
+                }
+                __syncwarp();
+                if (g < nHalves) {
+                    uint32_t f = sole | (todo & ~sw.drop[lane]);
+                    if (a.accumulate && f) all[row + g] |= f;
+                    if (s0) f |= out[row + g];
+                    out[row + g] = f;
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
-        for (int j = (int)lane; j < slots; j += 32) km[sw.list[j] >> 5] = 0u;
-        __syncwarp();
         distinct = warp_sum(distinct);
         if (lane == 0) a.aCount[p] = distinct;
     }
@@ -434,33 +530,38 @@ static int core_grid(int n, int warps) {
 }
 
 int launch_slot_sigs(const int32_t* topM, int D, int m, const int64_t* hubOff, const int32_t* hubLists, void* sig,
-                     uint64_t* multi, int W, int CT, cudaStream_t st) {
+                     cudaStream_t st) {
     const int total = 2 * D * m;
     k_slot_sigs<<<(total + 255) / 256, 256, 0, st>>>(topM, D, m, hubOff, hubLists, static_cast<int4*>(sig));
-    if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    k_multi_bits<<<(2 * D * W + 255) / 256, 256, 0, st>>>(static_cast<const int4*>(sig), D, m, W, CT, multi);
-    return cudaPeekAtLastError() == cudaSuccess ? 2 : -1;
-}
-
-int launch_core_dedupe(const CoreArgs& a, const void* sig, cudaStream_t st) {
-    const int warps = 8;
-    if (2 * a.k > kDdSlots || a.multi == nullptr) return -1;
-    const size_t sm = dedupe_warp_bytes((2 * a.nproj + 31) / 32) * warps;
-    if (sm > 48 * 1024 &&
-        cudaFuncSetAttribute(k_core_dedupe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
-        return -1;
-    k_core_dedupe<<<core_grid(a.n, warps), warps * 32, sm, st>>>(a, static_cast<const int4*>(sig));
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
-int launch_hub_masks(const CoreArgs& a, int32_t* hubIdx, int64_t* idxTmp, uint32_t* kMask, int64_t* scanTmp,
-                     int64_t* nHubsDev, cudaStream_t st) {
-    k_hub_flags<<<(a.n + 1 + 255) / 256, 256, 0, st>>>(a.hubOff, a.n, idxTmp);
+int launch_core_dedupe(const CoreArgs& a, cudaStream_t st) {
+    const int warps = 4;
+    // seen bits for every point that two lists can hold, whole 16 bytes
+    const int64_t most = std::min<int64_t>(a.n, (int64_t)a.nproj * a.m);
+    const int seenWords = (int)std::min<int64_t>(kDdSeenWords, (most + 127) / 128 * 4);
+    const size_t sm = dedupe_warp_bytes(seenWords, (2 * a.nproj + 31) / 32) * warps;
+    if (sm > 48 * 1024 &&
+        cudaFuncSetAttribute(k_core_dedupe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+        return -1;
+    const int perSm = (int)std::max<size_t>(1, std::min<size_t>(12, 224 * 1024 / (sm + 1024)));
+    const int blocks = std::min((a.n + warps - 1) / warps, sm_count() * perSm);
+    k_core_dedupe<<<blocks, warps * 32, sm, st>>>(a, seenWords);
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+
+int launch_hub_index(const CoreArgs& a, int32_t* hubIdx, int32_t* hubPoint, int32_t* multiIdx, uint32_t* kMask,
+                     int32_t* slotMulti, int32_t* slotHub, uint64_t* multi, unsigned long long* count,
+                     cudaStream_t st) {
+    k_hub_index<<<(a.n + 255) / 256, 256, 0, st>>>(a, hubIdx, hubPoint, multiIdx, count);
     if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    int r = launch_scan_i64(idxTmp, idxTmp, (size_t)a.n + 1, scanTmp, st);
-    if (r < 0) return -1;
-    k_hub_index<<<(a.n + 255) / 256, 256, 0, st>>>(a, idxTmp, hubIdx, kMask, nHubsDev);
-    return cudaPeekAtLastError() == cudaSuccess ? r + 2 : -1;
+    const int64_t hubs = std::min<int64_t>(a.n, (int64_t)2 * a.nproj * a.m);
+    k_hub_masks<<<(unsigned)((hubs + 7) / 8), 256, 0, st>>>(a, hubPoint, count, kMask);
+    if (cudaPeekAtLastError() != cudaSuccess) return -1;
+    k_slot_multi<<<(2 * a.nproj * a.W + 7) / 8, 256, 0, st>>>(a.topM, a.nproj, a.m, a.W, a.CT, multiIdx, hubIdx,
+                                                              slotMulti, slotHub, multi);
+    return cudaPeekAtLastError() == cudaSuccess ? 3 : -1;
 }
 
 int launch_core_finish(const CoreArgs& a, cudaStream_t st) {
