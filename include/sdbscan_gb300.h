@@ -118,7 +118,7 @@ sdb_status sdb_set_debug_limits(sdb_engine* e, int64_t stall_spins, int64_t queu
 
 /* Tile shape of the plain FP32 distance kernel (a tuning control; no
  * reference counterpart): 0 = the default: shape 3 where the distance has it
- * (Cosine, L1, L2) and the lists have 16 members or more on average, else 2 for topM in 41..50 and 1 otherwise, 1 = 128 x 64
+ * (all but JS) and the lists have 16 members or more on average, else 2 for topM in 41..50 and 1 otherwise, 1 = 128 x 64
  * tiles on 256 threads, 2 = 128 x 50 on 160 threads (32 dimensions per stage, 2
  * stages), 3 = the packed tile (two columns per instruction; 32, 40, 50 or 64
  * columns by topM; it keeps a copy of the candidate rows, and where that does

@@ -129,7 +129,7 @@ std::vector<DevBuf*> sdb_engine::all_bufs() {
             &noiseFlag, &noiseCores, &noisePts, &PcT, &numCore, &pairRound, &sngCols, &sngMult, &sngColOf, &sngExtras,
             &sngExtraPass, &sngMask, &rowDeg, &colCnt, &sngUb, &sngHeavy, &chunkOff, &tileKey, &keyOff, &tilePerm,
             &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask,
-            &multiIdx, &slotMulti, &slotHub, &hubPoint};
+            &multiIdx, &slotMulti, &slotHub, &hubPoint, &smallEntry};
 }
 
 // ---------------------------------------------------------------------------
@@ -305,6 +305,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
           ensure(hubPoint, sizeof(int32_t) * maxHubs) &&
           ensure(slotMulti, sizeof(int32_t) * (size_t)L * m) && ensure(slotHub, sizeof(int32_t) * (size_t)L * m);
     if (optics) ok &= ensure(sig, 16 * (size_t)L * m);
+    if (pairTiles && p.distance == SDB_CHI2) ok &= ensure(smallEntry, n);
     if (rff) ok &= ensure(E, sizeof(float) * (size_t)n * ker) && ensure(Rt, sizeof(float) * hostRt.size());
     if (optics || sweep) ok &= ensure(dists, sizeof(float) * (size_t)n * 2 * k * m);
     if (optics) ok &= ensure(coreDist, sizeof(float) * n);
@@ -371,6 +372,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     pa.scale = f32(scale);
     pa.compCosh = static_cast<const double*>(compCosh.ptr);
     pa.ln4 = ln4;
+    if (pairTiles && p.distance == SDB_CHI2) pa.small = static_cast<uint8_t*>(smallEntry.ptr);
     if (fuseXb) {
         if (!ensure(Xb, sizeof(uint16_t) * (size_t)n * ldb)) return SDB_ERR_NOMEM;
         pa.Xb = static_cast<uint16_t*>(Xb.ptr);
@@ -517,6 +519,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     da.nct = nct;
     da.TM = TMr;
     da.CT = CT;
+    da.small = static_cast<const uint8_t*>(smallEntry.ptr);
     da.cand = pairTiles ? f32(candT) : nullptr;
     da.eps = eps;
     if (sweep) da.eps = *std::max_element(sw->eps, sw->eps + sw->nEps);

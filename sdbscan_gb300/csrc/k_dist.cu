@@ -150,7 +150,7 @@ template <int DIST, int TX, int CN, int KT = TK, int NST = STAGES> int launch_di
 // for m in 41..50 and 64-column tiles otherwise.  1 = 128 x 64 (256 threads,
 // 32 dimensions per stage, 2 stages), 2 = 128 x 50 (160 threads, the same
 // stages).  Where the packed tile (3, k_dist_pair.cu) is asked for but not
-// available -- Chi2 and JS, the BF16 screening's fallback, a candidate copy
+// available -- JS, the BF16 screening's fallback, a candidate copy
 // that does not fit -- Cosine runs 128 x 50 with 16 dimensions in 4 stages
 // (the same shared memory, half the work between barriers and twice the loads
 // in flight; 3 % faster than 2 at 1M x 784, Chi2 2.5 % slower at 500K x 512).

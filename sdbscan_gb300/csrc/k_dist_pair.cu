@@ -1,6 +1,6 @@
 // Stage 4, the packed tile: candidate distances and the eps test of
 // rp_findCorePoints / rp_findCoreDist (src/sDbscan.cpp:243-359, :1323-1412)
-// for Cosine, L1 and L2 with the packed FP32 tile of pair_tile.cuh.
+// for Cosine, L1, L2 and Chi2 with the packed FP32 tile of pair_tile.cuh.
 //
 // Tile = (list l, TM member rows, CT candidate columns), as in k_dist.cu; the
 // candidate rows come from a dimension-major copy that k_cand_tiles writes
@@ -69,6 +69,7 @@ template <class S> struct PairSmem {
 // counts and (optionally) distances.
 template <int DIST, class S, int RM>
 __device__ __forceinline__ void pair_rows(const DistArgs& a, PairSmem<S>& sm, int rows, const float* cand, int ct) {
+    constexpr int kFinish = DIST == DIST_CHI2_ANY ? DIST_CHI2 : DIST;
     u64 acc[RM][S::CN / 2];
     pair_accumulate<DIST, S, RM>(a.Xt, a.ld, sm.rowLoad, cand, sm.As, sm.Bs, acc);
     if (!S::active(threadIdx.x)) return;
@@ -91,8 +92,8 @@ __device__ __forceinline__ void pair_rows(const DistArgs& a, PairSmem<S>& sm, in
             const int c = S::column(tx, j);
             float d0, d1;
             unpack2(acc[i][j], d0, d1);
-            d0 = dtile::finish<DIST>(d0);
-            d1 = dtile::finish<DIST>(d1);
+            d0 = dtile::finish<kFinish>(d0);
+            d1 = dtile::finish<kFinish>(d1);
             const int q0 = sm.colPoint[c], q1 = sm.colPoint[c + 1];
             const bool p0 = d0 <= a.eps && q0 >= 0 && q0 != p, p1 = d1 <= a.eps && q1 >= 0 && q1 != p;
             colPass[2 * j] += p0;
@@ -138,11 +139,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_dist_pair(DistArgs a) {
         sm.colCount[j] = 0;
     }
     if (tid == 0) sm.passTotal = 0;
-    __syncthreads();
+    bool small = false;  // Chi2: a row or a candidate of the tile has an entry below kChi2Small
+    if (DIST == DIST_CHI2) {
+        for (int i = tid; i < rows; i += kThreads) small |= a.small[sm.rowLoad[i]] != 0;
+        for (int j = tid; j < S::CT; j += kThreads) small |= sm.colPoint[j] >= 0 && a.small[sm.colPoint[j]] != 0;
+    }
+    small = __syncthreads_or(small);
 
     const float* cand = a.cand + ((size_t)l * a.nct + ct) * a.ld * S::CTP;
     const int need = (rows + S::RG - 1) / S::RG;  // rows per thread
-    if (need <= 2) pair_rows<DIST, S, 2>(a, sm, rows, cand, ct);
+    if (DIST == DIST_CHI2 && small) pair_rows<DIST_CHI2_ANY, S, S::RMAX>(a, sm, rows, cand, ct);
+    else if (need <= 2) pair_rows<DIST, S, 2>(a, sm, rows, cand, ct);
     else if (need <= 4) pair_rows<DIST, S, 4>(a, sm, rows, cand, ct);
     else if (S::RMAX == 6 || need <= 6) pair_rows<DIST, S, 6>(a, sm, rows, cand, ct);
     else pair_rows<DIST, S, S::RMAX>(a, sm, rows, cand, ct);
@@ -191,7 +198,7 @@ template <int DIST> int launch_pair_d(const DistArgs& a, cudaStream_t st) {
 // The columns per tile whose tiles take the least time for m candidates: the
 // cost of one column tile of each shape, in columns of the 64-wide one.
 int pair_tile_cols(int dist, int m) {
-    if (dist != DIST_COSINE && dist != DIST_L1 && dist != DIST_L2) return 0;
+    if (dist != DIST_COSINE && dist != DIST_L1 && dist != DIST_L2 && dist != DIST_CHI2) return 0;
     static const int shape[4][2] = {{64, 640}, {50, 542}, {40, 450}, {32, 370}};
     int best = 0, cols = 0;
     for (const auto& s : shape) {
@@ -227,6 +234,7 @@ int launch_dist_pair(const DistArgs& a, cudaStream_t st) {
         case DIST_COSINE: return launch_pair_d<DIST_COSINE>(a, st);
         case DIST_L1: return launch_pair_d<DIST_L1>(a, st);
         case DIST_L2: return launch_pair_d<DIST_L2>(a, st);
+        case DIST_CHI2: return launch_pair_d<DIST_CHI2>(a, st);
     }
     return -1;
 }

@@ -47,6 +47,11 @@ __device__ __forceinline__ u64 add2(u64 a, u64 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ u64 pack2(float lo, float hi) {
     u64 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -56,10 +61,47 @@ __device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// One dimension of two pairs: a the row's value in both halves, b the two
-// columns' values (negated for L1 / L2).
+// Chi2 terms x y / (x + y) of two pairs, correctly rounded, from a = -x and
+// b = -y: n = a b, D = a + b = -(x + y).  A reciprocal estimate, one Newton
+// step on it and one residual correction of the quotient (Markstein, IBM J.
+// Res. Dev. 34 (1990) 111): every operation but the estimate is packed.  Equal
+// to __fdiv_rn for all 2^46 pairs of significands (run through on the GPU), so
+// for all operands in range, and the range is kept by chi2_small: n is 0 or
+// >= 2^-100, which keeps the residual exact.  Where x + y < 2^-100, n is 0 and
+// so is the term, as long as the clamped D keeps the reciprocal finite.
+// The compiled division takes about 36 issue slots a term with its range
+// checks, this takes 6: 60K x 512, k = 10, m = 50, 27.7 -> 9.6 ms.  Bound: the
+// reciprocal unit (16 a cycle and SM, 6.2 ms) beside 8 FMA-pipe slots a term.
+constexpr float kChi2Small = 0x1p-50f;   // entries of (0, this) send a tile to the general term
+__device__ __forceinline__ u64 chi2_terms(u64 a, u64 b) {
+    const u64 n = mul2(a, b);
+    float d0, d1, y0, y1;
+    unpack2(add2(a, b), d0, d1);
+    d0 = fminf(d0, -0x1p-100f);
+    d1 = fminf(d1, -0x1p-100f);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(-d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(-d1));
+    const u64 D = pack2(d0, d1), y = pack2(y0, y1);
+    const u64 z = fma2(fma2(D, y, pack2(1.0f, 1.0f)), y, y);  // 1 / (x + y)
+    const u64 q = mul2(n, z);
+    return fma2(fma2(D, q, n), z, q);
+}
+
+// The general Chi2 term (any entries), a tile's slow form.
+constexpr int DIST_CHI2_ANY = 5;
+
+// One dimension of two pairs: a the row's value in both halves (negated for
+// Chi2), b the two columns' values (negated but for Cosine).
 template <int DIST> __device__ __forceinline__ u64 step2(u64 acc, u64 a, u64 b) {
     if (DIST == DIST_COSINE) return fma2(a, b, acc);
+    if (DIST == DIST_CHI2) return add2(acc, chi2_terms(a, b));
+    if (DIST == DIST_CHI2_ANY) {
+        float a0, a1, b0, b1, c0, c1;
+        unpack2(a, a0, a1);
+        unpack2(b, b0, b1);
+        unpack2(acc, c0, c1);
+        return pack2(dtile::acc_step<DIST_CHI2>(c0, -a0, -b0), dtile::acc_step<DIST_CHI2>(c1, -a1, -b1));
+    }
     const u64 t = add2(a, b);
     if (DIST == DIST_L2) return fma2(t, t, acc);
     float tl, th, cl, ch;  // L1
@@ -158,6 +200,29 @@ __device__ __forceinline__ void pair_accumulate(const float* __restrict__ Xt, in
                 }
             }
         };
+        if (DIST == DIST_CHI2 || DIST == DIST_CHI2_ANY) {
+            // a dimension at a time: four would be 30 KB of instructions
+#pragma unroll 1
+            for (int kk = 0; kk < kn; ++kk) {
+                const float* br = bs + kk * S::CTP;
+                u64 b[S::CN / 2];
+#pragma unroll
+                for (int q = 0; q < S::NQ; ++q) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(br + q * 4 * S::TX + 4 * tx);
+                    b[2 * q] = v.x;
+                    b[2 * q + 1] = v.y;
+                }
+                if (S::NP) b[S::CN / 2 - 1] = *reinterpret_cast<const u64*>(br + S::NQ * 4 * S::TX + 2 * tx);
+#pragma unroll
+                for (int i = 0; i < RM; ++i) {
+                    const float a = -as[i * S::RG * LDA + kk];
+                    const u64 a2 = pack2(a, a);
+#pragma unroll
+                    for (int j = 0; j < S::CN / 2; ++j) acc[i][j] = step2<DIST>(acc[i][j], a2, b[j]);
+                }
+            }
+            continue;
+        }
         // Cosine's widest tile unrolls a whole stage (30.0 against 32.7 ms at
         // 1M x 784) where enough stages follow to pay for fetching 27 KB of
         // instructions (50K x 128: 0.25 ms unrolled, 0.23 in the loop).  L1 /
