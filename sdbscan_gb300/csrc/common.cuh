@@ -96,8 +96,7 @@ struct ProjectArgs {
     int fhtDim, nproj, k;
     float* P;            // n x nproj projections out
     int32_t* topK;       // n x 2k out
-    float* chunkMax;     // G x nproj
-    float* chunkMin;     // G x nproj
+    uint32_t* chunkExt;  // G x nproj: (max v, max -v) of the chunk, BF16 rounded down, v in the low half
     int chunk;           // points per chunk (G = ceil(n / chunk))
     int chunkBase, chunkEnd;  // chunks this launch covers (chunkEnd 0: all G)
     int32_t* err;        // device flags: [0] negative input, [1] zero point
@@ -131,8 +130,7 @@ int launch_rff_tc(const void* Xb, const void* Rb, int n, int h, int ldb, float* 
 struct TopMArgs {
     const float* P;
     int n, nproj, m;
-    const float* chunkMax;
-    const float* chunkMin;
+    const uint32_t* chunkExt;  // ProjectArgs::chunkExt
     int G;
     float* thrMax;       // nproj
     float* thrMin;       // nproj

@@ -121,7 +121,7 @@ void sdb_engine::free_all() {
 }
 
 std::vector<DevBuf*> sdb_engine::all_bufs() {
-    return {&Xin, &Xt, &scale, &P, &topK, &chunkMax, &chunkMin, &thr, &cand, &candCount, &topM, &listCount,
+    return {&Xin, &Xt, &scale, &P, &topK, &chunkExt, &thr, &cand, &candCount, &topM, &listCount,
             &listOff, &members, &tileOff, &tileList, &hubCount, &hubOff, &hubLists, &masks, &inRaw,
             &aCount, &degree, &core, &parent, &border, &rootFlag, &labels, &nClusters, &scanTmp, &errFlags,
             &counters, &E, &Rt, &signs, &compCosh, &dists, &coreDist, &nbOff, &nbIdx, &nbDist, &nbFill, &hubIdx,
@@ -276,7 +276,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     if (!xOnDevice) ok &= ensure(Xin, sizeof(float) * (size_t)n * d);
     ok &= ensure(Xt, sizeof(float) * (size_t)n * ld) && ensure(scale, sizeof(float) * n) &&
           ensure(P, sizeof(float) * (size_t)n * D) && ensure(topK, sizeof(int32_t) * (size_t)n * 2 * k) &&
-          ensure(chunkMax, sizeof(float) * (size_t)G * D) && ensure(chunkMin, sizeof(float) * (size_t)G * D) &&
+          ensure(chunkExt, sizeof(uint32_t) * (size_t)G * D) &&
           ensure(thr, sizeof(float) * 2 * D) && ensure(cand, sizeof(uint64_t) * (size_t)L * cap) &&
           ensure(candCount, sizeof(int32_t) * L) && ensure(topM, sizeof(int32_t) * (size_t)D * 2 * m) &&
           ensure(listCount, sizeof(int64_t) * (L + 1)) && ensure(listOff, sizeof(int64_t) * (L + 1)) &&
@@ -363,8 +363,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     pa.k = k;
     pa.P = f32(P);
     pa.topK = i32(topK);
-    pa.chunkMax = f32(chunkMax);
-    pa.chunkMin = f32(chunkMin);
+    pa.chunkExt = static_cast<uint32_t*>(chunkExt.ptr);
     pa.chunk = chunk;
     pa.err = i32(errFlags);
     pa.ties = ctr + 0;
@@ -435,8 +434,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     ta.n = n;
     ta.nproj = D;
     ta.m = m;
-    ta.chunkMax = f32(chunkMax);
-    ta.chunkMin = f32(chunkMin);
+    ta.chunkExt = static_cast<const uint32_t*>(chunkExt.ptr);
     ta.G = G;
     ta.thrMax = f32(thr);
     ta.thrMin = f32(thr) + D;

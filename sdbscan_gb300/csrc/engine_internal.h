@@ -77,7 +77,7 @@ struct sdb_engine {
     std::vector<double> hostCosh;
 
     // device buffers (grow-only; kept across fits)
-    DevBuf Xin, Xt, scale, P, topK, chunkMax, chunkMin, thr, cand, candCount, topM, listCount, listOff,
+    DevBuf Xin, Xt, scale, P, topK, chunkExt, thr, cand, candCount, topM, listCount, listOff,
         members, tileOff, tileList, hubCount, hubOff, hubLists, masks, inRaw, aCount, degree, core, parent, border,
         rootFlag, labels, nClusters, scanTmp, errFlags, counters, E, Rt, signs, compCosh, dists, coreDist, nbOff,
         nbIdx, nbDist, nbFill, hubIdx, kMask, firstMasks, Xb, queue, sweepLabels, sweepNcl, sig, Rb, newMasks,

@@ -4,7 +4,8 @@
 //
 // Exact without a per-vector heap over n:
 //  1. The projection kernel leaves, for every chunk of points, the maximum
-//     and minimum projection onto each vector.  The m-th largest of the chunk
+//     and minimum projection onto each vector (as BF16 rounded away from the
+//     extreme, so still bounds of attained values).  The m-th largest of the chunk
 //     maxima is a value attained by m different points, so it is a lower
 //     bound T on the true m-th largest value (k_thresholds).
 //  2. One pass over the projections appends every (value, point) with value
@@ -49,52 +50,61 @@ __host__ __device__ inline int pow2_ceil(int x) {
     return p;
 }
 
-// One CTA per list (r, side): T = m-th largest key among the G chunk extremes
-// (0 when G < m), by a 4-pass 8-bit radix select over the keys staged in
-// shared memory.
-__global__ void k_thresholds(TopMArgs a) {
-    extern __shared__ uint32_t keys[];
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t selPrefix, selMask, selRank;
-    const int list = blockIdx.x;
-    const int r = list % a.nproj, side = list / a.nproj;
-    for (int g = threadIdx.x; g < a.G; g += blockDim.x) {
-        const float x = side == 0 ? a.chunkMax[(size_t)g * a.nproj + r] : -a.chunkMin[(size_t)g * a.nproj + r];
-        keys[g] = key_of(x);
-    }
-    if (threadIdx.x == 0) {
-        selPrefix = 0;
-        selMask = 0;
-        selRank = (uint32_t)a.m;  // rank (1-based, from the top) still to find inside the prefix
-    }
-    if (a.G < a.m) {
-        if (threadIdx.x == 0) (side == 0 ? a.thrMax : a.thrMin)[r] = __uint_as_float(0u);
-        return;
-    }
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-        __syncthreads();
-        const uint32_t pre = selPrefix, msk = selMask;
-        for (int g = threadIdx.x; g < a.G; g += blockDim.x) {
-            const uint32_t k = keys[g];
-            if ((k & msk) == pre) atomicAdd(&hist[(k >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t cum = 0, rank = selRank;
-            for (int b = 255; b >= 0; --b) {
-                if (cum + hist[b] >= rank) {
-                    selRank = rank - cum;
-                    selPrefix = pre | ((uint32_t)b << shift);
-                    selMask = msk | (255u << shift);
-                    break;
+// T of every list (r, side): the m-th largest chunk extreme, 0 with fewer than
+// m of them.  A CTA takes `cols` neighbouring vectors (32-byte row segments with
+// 8), folds `group` consecutive chunks into one (their maximum is attained
+// too) and keeps the results' 16-bit order-preserving keys in shared memory;
+// a warp then finds a list's m-th largest key by bisection, counting 16 times.
+// A 32-bit radix select with a histogram per list, and one CTA per column of
+// two float arrays, read 8 times the bytes, sent every key of a list (one
+// binade) at the same few bins and had one thread walk them: 104 us at any n
+// above 44K, D = 1024 (45 at 2K); this takes 30 (14), about half of it the
+// bisections.
+constexpr int kThrThreads = 512;
+__device__ __forceinline__ uint32_t key16(uint32_t b) { return (b & 0x8000u) ? ~b & 0xffffu : b | 0x8000u; }
+
+__global__ void __launch_bounds__(kThrThreads) k_thresholds(TopMArgs a, int cols, int group, int ng) {
+    extern __shared__ uint32_t keys[];  // ng x stride: (max key << 16) | min side's key
+    const int stride = cols | 1;
+    const int c = threadIdx.x & (cols - 1), r = blockIdx.x * cols + c, step = kThrThreads / cols;
+    if (r < a.nproj) {
+        for (int q = threadIdx.x / cols; q < ng; q += step) {
+            const int g1 = min(a.G, (q + 1) * group);
+            uint32_t hi = 0, lo = 0;
+            for (int g = q * group; g < g1; g += 8) {  // eight loads in flight (the last one again past the end)
+                uint32_t e[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) e[u] = __ldg(a.chunkExt + (size_t)min(g + u, g1 - 1) * a.nproj + r);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    hi = max(hi, key16(e[u] & 0xffffu));
+                    lo = max(lo, key16(e[u] >> 16));
                 }
-                cum += hist[b];
             }
+            keys[q * stride + c] = (hi << 16) | lo;
         }
-        __syncthreads();
     }
-    if (threadIdx.x == 0) (side == 0 ? a.thrMax : a.thrMin)[r] = __uint_as_float(selPrefix);  // raw key bits
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int l = threadIdx.x >> 5; l < 2 * cols; l += kThrThreads / 32) {
+        const int col = l >> 1, side = l & 1, rr = blockIdx.x * cols + col;
+        if (rr >= a.nproj) break;
+        uint32_t t = 0;
+        if (ng >= a.m) {
+            for (int bit = 15; bit >= 0; --bit) {
+                const uint32_t at = t | (1u << bit);
+                int cnt = 0;
+#pragma unroll 8
+                for (int q = lane; q < ng; q += 32) {
+                    const uint32_t k = keys[q * stride + col];
+                    cnt += (side ? k & 0xffffu : k >> 16) >= at;
+                }
+                if (warp_sum(cnt) >= a.m) t = at;
+            }
+            t = (t << 16) | (t & 0x8000u ? 0u : 0xffffu);  // the value's 32-bit key
+        }
+        if (lane == 0) (side ? a.thrMin : a.thrMax)[rr] = __uint_as_float(t);  // raw key bits
+    }
 }
 
 // A block takes kCollectRows consecutive points; a thread takes 4
@@ -278,11 +288,16 @@ __global__ void k_fallback(TopMArgs a) {
 }  // namespace
 
 int launch_topm_thresholds(const TopMArgs& a, cudaStream_t st) {
-    const size_t sm = sizeof(uint32_t) * (size_t)a.G;
+    // 912 groups or 4m: enough that the m-th largest is close to the m-th value
+    const int group = std::max(1, a.G / std::max(912, 4 * a.m));
+    const int ng = (a.G + group - 1) / group;
+    int cols = 8;
+    while (cols > 1 && sizeof(uint32_t) * (size_t)ng * (cols | 1) > 100 * 1024) cols >>= 1;
+    const size_t sm = sizeof(uint32_t) * (size_t)ng * (cols | 1);
     if (sm > 48 * 1024 &&
         cudaFuncSetAttribute(k_thresholds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
         return -1;
-    k_thresholds<<<2 * a.nproj, 256, sm, st>>>(a);
+    k_thresholds<<<(a.nproj + cols - 1) / cols, kThrThreads, sm, st>>>(a, cols, group, ng);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 

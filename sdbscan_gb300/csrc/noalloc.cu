@@ -11,13 +11,14 @@
 // from one file-scope __device__ array, g_topmScratch, below.
 //
 // Limits (from the fixed scratch size): n_proj <= 1024, topM <= 64.  The
-// array (about 12 MiB) is reserved on every GPU that loads this library, for
+// array (about 10 MiB) is reserved on every GPU that loads this library, for
 // as long as the library stays loaded.  All calls share it: two calls that
 // overlap on the GPU (different streams, or different host threads) race and
 // must not be issued.  Each call zeroes the counters it needs, so successive
 // calls do not see the previous call's state.  The boundary-tie count and the
 // internal-error flag that a fit reports are kept in the array but not
 // returned by this entry point.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -36,9 +37,8 @@ constexpr int kLists = 2 * kMaxProj;
 
 // Scratch layout, in bytes from the start of the array.
 constexpr size_t kOffCand = 0;                                                    // kLists * kCap u64
-constexpr size_t kOffChunkMax = kOffCand + sizeof(uint64_t) * kLists * kCap;      // kMaxChunks * kMaxProj f32
-constexpr size_t kOffChunkMin = kOffChunkMax + sizeof(float) * kMaxChunks * kMaxProj;
-constexpr size_t kOffThr = kOffChunkMin + sizeof(float) * kMaxChunks * kMaxProj;  // 2 * kMaxProj f32
+constexpr size_t kOffChunkExt = kOffCand + sizeof(uint64_t) * kLists * kCap;      // kMaxChunks * kMaxProj u32
+constexpr size_t kOffThr = kOffChunkExt + sizeof(uint32_t) * kMaxChunks * kMaxProj;  // 2 * kMaxProj f32
 constexpr size_t kOffCount = kOffThr + sizeof(float) * 2 * kMaxProj;              // kLists i32
 constexpr size_t kOffFlags = kOffCount + sizeof(int32_t) * kLists;                // 4 i32 + 2 u64
 constexpr size_t kScratchBytes = kOffFlags + 64;
@@ -51,8 +51,9 @@ void* g_scratchPtr[64] = {};
 
 // Column maxima / minima of the projections over `chunk` consecutive points:
 // the chunk extremes the top-m thresholds are built from.
-__global__ void k_chunk_extremes(const float* __restrict__ P, int n, int nproj, int chunk, float* __restrict__ cmax,
-                                 float* __restrict__ cmin) {
+// In the form k_project leaves them: (max, max of -v) as BF16 rounded down.
+__global__ void k_chunk_extremes(const float* __restrict__ P, int n, int nproj, int chunk,
+                                 uint32_t* __restrict__ ext) {
     const int g = blockIdx.x;
     const int p0 = g * chunk, p1 = min(n, p0 + chunk);
     for (int r = threadIdx.x; r < nproj; r += blockDim.x) {
@@ -62,8 +63,10 @@ __global__ void k_chunk_extremes(const float* __restrict__ P, int n, int nproj, 
             mx = fmaxf(mx, v);
             mn = fminf(mn, v);
         }
-        cmax[(size_t)g * nproj + r] = mx;
-        cmin[(size_t)g * nproj + r] = mn;
+        __nv_bfloat162 b;
+        b.x = __float2bfloat16_rd(mx);
+        b.y = __float2bfloat16_rd(-mn);
+        ext[(size_t)g * nproj + r] = *reinterpret_cast<const uint32_t*>(&b);
     }
 }
 
@@ -100,8 +103,8 @@ extern "C" sdb_status sdb_topm_noalloc(const float* proj_device, int32_t n_point
     a.n = n_points;
     a.nproj = n_proj;
     a.m = topM;
-    a.chunkMax = reinterpret_cast<float*>(base + kOffChunkMax);
-    a.chunkMin = reinterpret_cast<float*>(base + kOffChunkMin);
+    uint32_t* ext = reinterpret_cast<uint32_t*>(base + kOffChunkExt);
+    a.chunkExt = ext;
     a.G = G;
     a.thrMax = reinterpret_cast<float*>(base + kOffThr);
     a.thrMin = a.thrMax + n_proj;
@@ -115,8 +118,7 @@ extern "C" sdb_status sdb_topm_noalloc(const float* proj_device, int32_t n_point
     if (cudaMemsetAsync(base + kOffCount, 0, sizeof(int32_t) * 2 * n_proj, st) != cudaSuccess ||
         cudaMemsetAsync(base + kOffFlags, 0, 64, st) != cudaSuccess)
         return SDB_ERR_CUDA;
-    k_chunk_extremes<<<G, 256, 0, st>>>(proj_device, n_points, n_proj, chunk, const_cast<float*>(a.chunkMax),
-                                         const_cast<float*>(a.chunkMin));
+    k_chunk_extremes<<<G, 256, 0, st>>>(proj_device, n_points, n_proj, chunk, ext);
     if (cudaPeekAtLastError() != cudaSuccess) return SDB_ERR_CUDA;
     if (sdb::launch_topm_thresholds(a, st) < 0 || sdb::launch_topm_collect(a, st) < 0 ||
         sdb::launch_topm_select(a, st) < 0)
