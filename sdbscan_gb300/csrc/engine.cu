@@ -49,6 +49,9 @@ constexpr int kSuperChunk = 8;
 constexpr size_t kMaxCandBytes = (size_t)8 << 30;
 constexpr int kMinCandMembers = 16;
 
+// Host input per upload segment.
+constexpr size_t kSegBytes = (size_t)256 << 20;
+
 size_t kTcKeys(int n, int L) {
     const int nChunks = (n + 4095) / 4096;
     return (size_t)((nChunks + kSuperChunk - 1) / kSuperChunk) * L + 1;
@@ -401,7 +404,13 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
         pa.do_transform = 0;
     }
     if (overlapUpload) {
-        const int segs = std::min(kUploadSegs, G);
+        // one segment per kSegBytes: each segment's kernels start and drain on a
+        // part of the points only, about 0.08 ms a segment, and the link brings
+        // 190 GB/s.  Projection stage with 16 segments against this rule: 40K x
+        // 256 (41 MB) 1.58 and 0.50 ms, 70K x 784 (220 MB) 4.43 and 1.79, 200K x
+        // 784 (627 MB) 7.86 and 4.75; 1M x 784 keeps twelve.
+        const size_t xBytes = sizeof(float) * (size_t)n * d;
+        const int segs = (int)std::min<size_t>(std::min(kUploadSegs, G), std::max<size_t>(1, xBytes / kSegBytes));
         SDB_CK(cudaEventRecord(segEv[kUploadSegs], st));  // Xin is free once the stream got here
         for (int c = 0; c < kCopyStreams; ++c) SDB_CK(cudaStreamWaitEvent(copyStream[c], segEv[kUploadSegs], 0));
         // every copy is queued before the first projection launch, so a delay
