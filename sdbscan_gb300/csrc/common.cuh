@@ -336,6 +336,24 @@ int launch_uf_init(int32_t* parent, int32_t* border, int n, cudaStream_t st);
 int launch_uf_compress(const ClusterArgs& a, cudaStream_t st);
 int launch_cluster_labels(const ClusterArgs& a, cudaStream_t st);
 
+// The sOPTICS ordering's floods from the symmetric neighbour lists (k_order.cu).
+struct CsrArgs {
+    int n;
+    const uint8_t* core;
+    const float* coreDist;
+    const int64_t* off;    // n + 1
+    const int32_t* idx;
+    const float* dist;
+    int32_t* parent;       // n, parent[p] = p on entry
+    int32_t* start;        // n out: the point whose turn in the outer loop emits p
+    // the lists for the host: point p's at place newId[p], core points' only
+    const int32_t* newId;  // n
+    int64_t* edgeOff;      // n + 1 out
+    uint2* edges;          // (newId of the neighbour, key of max(core distance, distance)) out
+};
+int launch_csr_starts(const CsrArgs& a, cudaStream_t st);
+int launch_csr_edges(const CsrArgs& a, int64_t* scanTmp, cudaStream_t st);
+
 // sngDbscan / sngOptics (src/sDbscan.cpp:416-504, :1484-1583) over one
 // shared sample of columns: every point is a row, every distinct sampled
 // point a column.

@@ -132,7 +132,8 @@ std::vector<DevBuf*> sdb_engine::all_bufs() {
             &noiseFlag, &noiseCores, &noisePts, &PcT, &numCore, &pairRound, &sngCols, &sngMult, &sngColOf, &sngExtras,
             &sngExtraPass, &sngMask, &rowDeg, &colCnt, &sngUb, &sngHeavy, &chunkOff, &tileKey, &keyOff, &tilePerm,
             &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask,
-            &multiIdx, &slotMulti, &slotHub, &hubPoint, &smallEntry};
+            &multiIdx, &slotMulti, &slotHub, &hubPoint, &smallEntry,
+            &floodStart, &newId, &edgeOff, &edges};
 }
 
 // ---------------------------------------------------------------------------

@@ -84,19 +84,18 @@ struct sdb_engine {
         coreEps, sampleFlag, noiseFlag, noiseCores, noisePts, PcT, numCore, pairRound, sngCols, sngMult, sngColOf,
         sngExtras, sngExtraPass, sngMask, rowDeg, colCnt, sngUb, sngHeavy, chunkOff, tileKey, keyOff, tilePerm, Cb, candT,
         tileKeyTc, keyOffTc, tilePermTc, sngWords, hashOffB, hashIdB, hashDistB, sqNorm, multiMask, multiIdx, slotMulti,
-        slotHub, hubPoint, smallEntry;
+        slotHub, hubPoint, smallEntry, floodStart, newId, edgeOff, edges;
 
     // results
     bool haveLabels = false, haveOptics = false, haveFit = false, lastOptics = false;
     bool lastSng = false;  // the last fit was sngDbscan / sngOptics (no index state)
     std::vector<int32_t> hostOrdering;
     std::vector<float> hostReach;
-    // the sOPTICS neighbour lists, core distances and core flags downloaded
-    // for the host ordering
+    // the sOPTICS neighbour lists downloaded for the host ordering, and its
+    // per-point work arrays
     HostBuf<int64_t> stageOff;
-    HostBuf<int32_t> stageIdx;
-    HostBuf<float> stageDist, stageCd;
-    HostBuf<uint8_t> stageCore;
+    HostBuf<uint64_t> stageEdge;
+    HostBuf<int32_t> stageInt;
     int32_t* hostErr = nullptr;
     unsigned long long* hostCounters = nullptr;
     int launchCount = 0;

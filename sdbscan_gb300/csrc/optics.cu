@@ -2,16 +2,22 @@
 // GPU (rp_findCoreDist, src/sDbscan.cpp:1314-1474), then the ordering and
 // reachability (formOptics_scikit, src/sDbscan.cpp:1588-1703).
 //
-// The ordering is a priority flood: each step pops the unprocessed point of
-// least reachability, so it is inherently sequential.  It runs here in host
-// C++ over the CSR the GPU produced.  Ties between equal reachability values,
+// The ordering is a sequence of priority floods: each step pops the
+// unprocessed point of least reachability, so a flood is inherently
+// sequential, but the floods are independent of one another (k_order.cu).
+// They run here in host C++, one host thread per flood at a time, over lists
+// the GPU has regrouped by flood.  Ties between equal reachability values,
 // which the reference's value-only heap resolves by heap order, are resolved
 // by the smaller point id, so the ordering does not depend on the order of
 // the neighbour lists.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <exception>
 #include <new>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -28,85 +34,95 @@ using namespace sdb;
 
 namespace {
 
-// formOptics_scikit with (reachability, point id) order.  reach[] holds
-// NEG_INF (-2^31) for points never reached (src/sDbscan.cpp:1590).  The
-// reference keeps a lazy-deletion heap (Min_PQ_Pair seedSet, :1609); here the
-// seed queue is an indexed 4-ary min-heap on (reach, id) with decrease-key,
-// each unprocessed point in it at most once: the same pop sequence as a lazy
-// heap with that order, with fewer heap operations.
-void form_optics(int n, const uint8_t* core, const float* coreDist, const int64_t* off, const int32_t* idx,
-                 const float* dist, int32_t* ordering, float* reach) {
-    std::fill(reach, reach + n, kNegInfReach);
-    std::vector<uint8_t> done(n, 0);
-    std::vector<int32_t> pos(n, -1), heap;
-    heap.reserve(4096);
-    auto less = [&](int a, int b) { return reach[a] < reach[b] || (reach[a] == reach[b] && a < b); };
-    auto sift_up = [&](int i) {
-        const int y = heap[i];
-        while (i > 0) {
-            const int par = (i - 1) >> 2;
-            if (!less(y, heap[par])) break;
-            heap[i] = heap[par];
-            pos[heap[i]] = i;
-            i = par;
-        }
-        heap[i] = y;
-        pos[y] = i;
-    };
-    auto sift_down = [&](int i) {
-        const int y = heap[i], sz = (int)heap.size();
-        while (true) {
-            const int c0 = 4 * i + 1;
-            if (c0 >= sz) break;
-            int b = c0;
-            for (int c = c0 + 1; c < std::min(c0 + 4, sz); ++c)
-                if (less(heap[c], heap[b])) b = c;
-            if (!less(heap[b], y)) break;
-            heap[i] = heap[b];
-            pos[heap[i]] = i;
-            i = b;
-        }
-        heap[i] = y;
-        pos[y] = i;
-    };
-    int64_t no = 0;
-    auto relax = [&](int x) {
-        const float cd = coreDist[x];
-        for (int64_t t = off[x]; t < off[x + 1]; ++t) {
-            const int y = idx[t];
-            if (done[y]) continue;
-            const float r = std::max(cd, dist[t]);
-            if (reach[y] == kNegInfReach) {
-                reach[y] = r;
-                heap.push_back(y);
-                sift_up((int)heap.size() - 1);
-            } else if (reach[y] > r) {
-                reach[y] = r;
-                sift_up(pos[y]);
+struct Edge {
+    uint32_t to, key;  // neighbour's number, order-preserving key of max(core distance, distance)
+};
+
+constexpr uint32_t kDone = 0, kUnreached = 0xffffffffu;  // no float has these keys
+
+// The inverse of key_of (common.cuh).
+float key_value(uint32_t k) {
+    const uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+    float f;
+    std::memcpy(&f, &u, sizeof f);
+    return f;
+}
+
+struct Flood {
+    int64_t entries;         // of its lists
+    int first, last, start;  // its points' numbers [first, last) and the start's
+};
+
+// The floods of formOptics_scikit.  The points are numbered flood by flood
+// (the outer loop's order), by point id within a flood.  best[y] is y's key:
+// kUnreached, the key of its reachability while it is a seed, kDone after.
+// The seed queue (Min_PQ_Pair seedSet, src/sDbscan.cpp:1609, a lazy-deletion
+// heap there) is an indexed 4-ary min-heap of (key, number) words with
+// decrease-key: the same pop sequence in fewer heap operations, and one
+// comparison of words is the order by reachability, then id.
+struct Floods {
+    const int64_t* edgeOff;
+    const Edge* edges;
+    const int32_t* orig;  // number -> point id
+    uint32_t* best;
+    int32_t* pos;
+    int32_t* ordering;
+    float* reach;
+
+    void run(int first, int last, int start, std::vector<uint64_t>& heap) const {
+        heap.resize((size_t)(last - first));
+        uint64_t* h = heap.data();
+        int size = 0, out = first;
+        for (int y = first; y < last; ++y) best[y] = kUnreached;
+        auto relax = [&](int x) {
+            const Edge* const end = edges + edgeOff[x + 1];
+            for (const Edge* e = edges + edgeOff[x]; e != end; ++e) {
+                const uint32_t old = best[e->to];
+                if (e->key >= old) continue;  // done, or reached as near already
+                best[e->to] = e->key;
+                const uint64_t word = (uint64_t)e->key << 32 | e->to;
+                int i = old == kUnreached ? size++ : pos[e->to];
+                while (i > 0) {
+                    const int par = (i - 1) >> 2;
+                    if (word >= h[par]) break;
+                    h[i] = h[par];
+                    pos[(uint32_t)h[i]] = i;
+                    i = par;
+                }
+                h[i] = word;
+                pos[e->to] = i;
             }
-        }
-    };
-    for (int p = 0; p < n; ++p) {
-        if (done[p]) continue;
-        done[p] = 1;
-        ordering[no++] = p;
-        if (!core[p]) continue;
-        relax(p);
-        while (!heap.empty()) {
-            const int y = heap[0];
-            const int last = heap.back();
-            heap.pop_back();
-            if (!heap.empty()) {
-                heap[0] = last;
-                sift_down(0);
+        };
+        best[start] = kDone;
+        ordering[out++] = orig[start];
+        reach[orig[start]] = kNegInfReach;
+        relax(start);
+        while (size > 0) {
+            const uint64_t top = h[0];
+            const uint64_t word = h[--size];
+            if (size > 0) {
+                int i = 0;
+                for (int c = 1; c < size; c = 4 * i + 1) {
+                    int b = c;
+                    const int end = std::min(c + 4, size);
+                    for (int k = c + 1; k < end; ++k)
+                        if (h[k] < h[b]) b = k;
+                    if (h[b] >= word) break;
+                    h[i] = h[b];
+                    pos[(uint32_t)h[i]] = i;
+                    i = b;
+                }
+                h[i] = word;
+                pos[(uint32_t)word] = i;
             }
-            pos[y] = -1;
-            done[y] = 1;
-            ordering[no++] = y;
-            if (core[y]) relax(y);
+            const int y = (int)(uint32_t)top;
+            best[y] = kDone;
+            ordering[out++] = orig[y];
+            reach[orig[y]] = key_value((uint32_t)(top >> 32));
+            relax(y);
         }
     }
-}
+};
 
 }  // namespace
 
@@ -140,38 +156,119 @@ sdb_status sdb_engine::optics_stage(const CoreArgs& ca, int& launches) {
     return optics_order(total);
 }
 
-// Downloads the CSR neighbour lists (nbOff / nbIdx / nbDist), core flags and
-// core distances of the last fit and runs the ordering on the host.
-// The staging buffers are kept across fits and not zero-filled: a fresh,
-// zeroed buffer per fit costs a memset and first-touch page faults over the
-// whole list (hundreds of MB at 500K points) before the copy overwrites it.
+// The ordering and reachability from the neighbour lists of the last fit
+// (nbOff / nbIdx / nbDist), core flags and core distances.  The lists' staging
+// buffer is kept across fits and not zero-filled: a fresh, zeroed buffer per
+// fit costs a memset and first-touch page faults over the whole list (hundreds
+// of MB at 500K points) before the copy overwrites it.
+// 50K x 784, 5 M list entries in ten floods: 27.9 ms for one serial flood over
+// the downloaded lists, 2.8 with the floods apart (16 host cores).
 sdb_status sdb_engine::optics_order(int64_t total) {
     cudaStream_t st = stream;
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
+    if (!ensure(parent, sizeof(int32_t) * n) || !ensure(border, sizeof(int32_t) * n) ||
+        !ensure(floodStart, sizeof(int32_t) * n) || !ensure(newId, sizeof(int32_t) * n) ||
+        !ensure(edgeOff, sizeof(int64_t) * (n + 1)) || !ensure(edges, sizeof(Edge) * std::max<int64_t>(total, 1)))
+        return SDB_ERR_NOMEM;
+    CsrArgs a{};
+    a.n = n;
+    a.core = static_cast<const uint8_t*>(core.ptr);
+    a.coreDist = f32(coreDist);
+    a.off = i64(nbOff);
+    a.idx = i32(nbIdx);
+    a.dist = f32(nbDist);
+    a.parent = i32(parent);
+    a.start = i32(floodStart);
+    a.newId = i32(newId);
+    a.edgeOff = i64(edgeOff);
+    a.edges = static_cast<uint2*>(edges.ptr);
+    if (launch_uf_init(i32(parent), i32(border), n, st) < 0 || launch_csr_starts(a, st) < 0)
+        return fail(SDB_ERR_CUDA, "flood launch failed");
+    int32_t *hStart = nullptr, *hNew = nullptr, *hOrig = nullptr, *hPos = nullptr, *hFirst = nullptr;
+    uint32_t* hBest = nullptr;
     int64_t* hOff = nullptr;
-    int32_t* hIdx = nullptr;
-    float *hDist = nullptr, *hCd = nullptr;
-    uint8_t* hCore = nullptr;
+    Edge* hEdges = nullptr;
     try {
+        int32_t* w = stageInt.get((size_t)n * 6 + 1);
+        hStart = w;
+        hNew = w + n;
+        hOrig = w + 2 * (size_t)n;
+        hPos = w + 3 * (size_t)n;
+        hBest = reinterpret_cast<uint32_t*>(w + 4 * (size_t)n);
+        hFirst = w + 5 * (size_t)n;
         hOff = stageOff.get((size_t)n + 1);
-        hIdx = stageIdx.get((size_t)std::max<int64_t>(total, 1));
-        hDist = stageDist.get((size_t)std::max<int64_t>(total, 1));
-        hCd = stageCd.get((size_t)n);
-        hCore = stageCore.get((size_t)n);
-        hostOrdering.assign(n, 0);
-        hostReach.assign(n, 0.0f);
+        hEdges = reinterpret_cast<Edge*>(stageEdge.get((size_t)std::max<int64_t>(total, 1)));
+        hostOrdering.resize(n);
+        hostReach.resize(n);
     } catch (const std::bad_alloc&) {
         return fail(SDB_ERR_NOMEM, "host memory for the sOPTICS neighbour lists");
     }
-    e = cudaMemcpyAsync(hOff, nbOff.ptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && total)
-        e = cudaMemcpyAsync(hIdx, nbIdx.ptr, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && total)
-        e = cudaMemcpyAsync(hDist, nbDist.ptr, sizeof(float) * total, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hCd, coreDist.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hCore, core.ptr, n, cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(hStart, floodStart.ptr, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(e, "flood starts");
+    // number the points by (start, id): a counting sort that keeps the ids' order
+    std::fill(hFirst, hFirst + n + 1, 0);
+    for (int p = 0; p < n; ++p) ++hFirst[hStart[p] + 1];
+    for (int p = 0; p < n; ++p) hFirst[p + 1] += hFirst[p];
+    for (int p = n - 1; p >= 0; --p) {
+        const int q = --hFirst[hStart[p] + 1];
+        hNew[p] = q;
+        hOrig[q] = p;
+    }
+    e = cudaMemcpyAsync(newId.ptr, hNew, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return cuda_fail(e, "flood numbers");
+    if (launch_csr_edges(a, i64(scanTmp), st) < 0) return fail(SDB_ERR_CUDA, "flood list launch failed");
+    e = cudaMemcpyAsync(hOff, edgeOff.ptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const int64_t kept = e == cudaSuccess ? hOff[n] : 0;
+    if (e == cudaSuccess && kept)
+        e = cudaMemcpyAsync(hEdges, edges.ptr, sizeof(Edge) * kept, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "neighbour list download");
-    form_optics(n, hCore, hCd, hOff, hIdx, hDist, hostOrdering.data(), hostReach.data());
+
+    const Floods fl{hOff, hEdges, hOrig, hBest, hPos, hostOrdering.data(), hostReach.data()};
+    try {
+        std::vector<Flood> order;  // of more than one point
+        for (int q = 0; q < n;) {
+            const int s = hStart[hOrig[q]];
+            int last = q + 1;
+            while (last < n && hStart[hOrig[last]] == s) ++last;
+            if (last == q + 1) {
+                hostOrdering[q] = s;
+                hostReach[s] = kNegInfReach;
+            } else {
+                order.push_back(Flood{hOff[last] - hOff[q], q, last, hNew[s]});
+            }
+            q = last;
+        }
+        std::sort(order.begin(), order.end(), [](const Flood& x, const Flood& y) { return x.entries > y.entries; });
+        std::atomic<size_t> next{0};
+        std::atomic<bool> failed{false};
+        auto work = [&]() {
+            try {
+                std::vector<uint64_t> heap;
+                for (size_t t; (t = next.fetch_add(1)) < order.size();) {
+                    fl.run(order[t].first, order[t].last, order[t].start, heap);
+                }
+            } catch (...) {
+                failed = true;
+            }
+        };
+        // the largest floods first; a thread more for every 200K list entries
+        // (starting one takes 0.06 ms)
+        const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+        const size_t threads = std::min<size_t>({(size_t)hw, order.size(), (size_t)(kept / 200000) + 1, (size_t)32});
+        std::vector<std::thread> helpers;
+        try {
+            for (size_t t = 1; t < threads; ++t) helpers.emplace_back(work);
+        } catch (const std::exception&) {
+            // fewer threads than wanted: the ones that started and this one do it all
+        }
+        work();
+        for (std::thread& t : helpers) t.join();
+        if (failed) return fail(SDB_ERR_NOMEM, "host memory for the sOPTICS seed queue");
+    } catch (const std::bad_alloc&) {
+        return fail(SDB_ERR_NOMEM, "host memory for the sOPTICS floods");
+    }
     return SDB_OK;
 }

@@ -1,0 +1,54 @@
+"""The sOPTICS ordering as independent floods (csrc/k_order.cu, optics.cu)
+against the oracle's one sequential flood: non-core points between two
+clusters, non-core points whose turn comes before their cluster's smallest
+core point, one flood, none, and enough list entries for several threads."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _clusters(n, d, c, spread, seed, order):
+    """c clusters whose edges overlap; order "edges_first" gives the points far
+    from their centre the small ids, "edges_last" the large ones."""
+    rng = np.random.default_rng(seed)
+    centre = rng.standard_normal((c, d))
+    y = rng.integers(0, c, n)
+    r = rng.random(n) ** 0.5
+    z = rng.standard_normal((n, d))
+    X = centre[y] + spread * r[:, None] * z
+    if order != "mixed":
+        i = np.argsort(-r if order == "edges_first" else r, kind="stable")
+        X = X[i]
+    return np.ascontiguousarray(X.astype(np.float32))
+
+
+@pytest.mark.parametrize("n,d,c,spread,eps,minPts,order", [
+    (3000, 8, 6, 0.6, 0.05, 8, "edges_first"),
+    (3000, 8, 6, 0.6, 0.05, 8, "edges_last"),
+    (20000, 16, 12, 0.35, 0.06, 10, "mixed"),   # millions of list entries, several threads
+    (4000, 6, 1, 0.3, 0.3, 5, "mixed"),         # one flood
+    (1500, 12, 5, 0.5, 0.001, 5, "mixed"),      # no core point
+    (40, 5, 3, 0.4, 0.1, 3, "edges_first"),
+])
+def test_ordering_matches_oracle(n, d, c, spread, eps, minPts, order):
+    from oracle.oracle import Port, build_port
+    from sdbscan_gb300 import capi
+    build_port()
+    X = _clusters(n, d, c, spread, n + c, order)
+    e = capi.Engine(n, d)
+    e.set_params(n_proj=256, topK=8, topM=min(60, n), random_seed=4)
+    e.fit_soptics(X, eps, minPts)
+    ordering, reach = e.optics()
+    core, _ = e.core()
+    cd = e.core_dist()
+    o_order, o_reach, o_core, o_cd, _ = Port().fit_soptics(X, eps, minPts, n_proj=256, topK=8, topM=min(60, n), seed=4,
+                                                           threads=4, tie_mode=1)
+    np.testing.assert_array_equal(core, o_core)
+    np.testing.assert_array_equal(cd, o_cd)
+    np.testing.assert_array_equal(ordering, o_order)
+    np.testing.assert_array_equal(reach, o_reach)
+    e.fit_soptics(X, eps, minPts)  # again on the same engine
+    np.testing.assert_array_equal(e.optics()[0], o_order)
+    np.testing.assert_array_equal(e.optics()[1], o_reach)
+    e.close()
