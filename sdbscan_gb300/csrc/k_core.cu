@@ -86,24 +86,25 @@ __global__ void __launch_bounds__(256) k_hub_index(CoreArgs a, int32_t* __restri
     if (lists > 0) hubPoint[h] = p;
 }
 
-// The hubs' list masks, a warp per hub, a word per lane.
-__global__ void __launch_bounds__(256) k_hub_masks(CoreArgs a, const int32_t* __restrict__ hubPoint,
-                                                   const unsigned long long* __restrict__ count,
-                                                   uint32_t* __restrict__ kMask) {
+// The hubs' list masks, a warp per hub, the mask put together in shared memory.
+constexpr int kHmWarps = 8, kHmWords = 128;  // 2D <= 4096 lists
+__global__ void __launch_bounds__(32 * kHmWarps) k_hub_masks(CoreArgs a, const int32_t* __restrict__ hubPoint,
+                                                             const unsigned long long* __restrict__ count,
+                                                             uint32_t* __restrict__ kMask) {
+    __shared__ uint32_t mask[kHmWarps][kHmWords];
     const int h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (h >= (int)__ldg(count)) return;
     const int lane = (int)lane_id(), words = (2 * a.nproj + 31) / 32, slots = 2 * a.k;
+    uint32_t* m = mask[threadIdx.x >> 5];
     const int32_t* tk = a.topK + (size_t)__ldg(hubPoint + h) * slots;
-    const int lA = lane < slots ? __ldg(tk + lane) + (lane >= a.k ? a.nproj : 0) : 0;
-    const int lB = lane + 32 < slots ? __ldg(tk + lane + 32) + (lane + 32 >= a.k ? a.nproj : 0) : 0;
-    for (int w0 = 0; w0 < words; w0 += 32) {
-        uint32_t bits = 0;
-        for (int j = 0; j < slots; ++j) {
-            const int l = __shfl_sync(0xffffffffu, j < 32 ? lA : lB, j & 31);
-            if (l >> 5 == w0 + lane) bits |= 1u << (l & 31);
-        }
-        if (w0 + lane < words) kMask[(size_t)h * words + w0 + lane] = bits;
+    for (int w = lane; w < words; w += 32) m[w] = 0u;
+    __syncwarp();
+    for (int j = lane; j < slots; j += 32) {
+        const int l = __ldg(tk + j) + (j >= a.k ? a.nproj : 0);
+        atomicOr(m + (l >> 5), 1u << (l & 31));
     }
+    __syncwarp();
+    for (int w = lane; w < words; w += 32) kMask[(size_t)h * words + w] = m[w];
 }
 
 // A warp per (list, word): slotMulti and slotHub = multiIdx and hubIdx of the
@@ -271,6 +272,67 @@ __host__ __device__ constexpr size_t dedupe_warp_bytes(int seenWords, int maskWo
     return (sizeof(uint32_t) * ((size_t)seenWords + maskWords) + sizeof(DedupeWarp) + 15) / 16 * 16;
 }
 
+// A point of at most 32 passing pairs, a pair per lane: repeats are lanes of
+// the same candidate (no seen bits to clear: 150K x 256 L2, m = 100, core stage
+// 266 -> 145 us).  Returns the number of distinct candidates; the point's
+// output words are cleared already.  pairs: of this lane's 16-byte pieces.  (Not
+// inlined: it costs the dense path registers.)
+__device__ __noinline__ int dedupe_sparse(const CoreArgs& a, DedupeWarp& sw, const uint32_t* listMask, int p, int np,
+                                          int pairs, int allPairs) {
+    const int lane = (int)lane_id(), slots = 2 * a.k, maskWords = (2 * a.nproj + 31) / 32;
+    const size_t row = (size_t)p * 2 * slots * a.W;
+    const uint4* row4 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(a.masks) + row);
+    uint32_t* item = reinterpret_cast<uint32_t*>(sw.item);
+    int at = pairs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    at -= pairs;
+    for (int t = lane; pairs > 0; t += 32) {
+        const uint4 v = __ldg(row4 + t);
+        const uint32_t halves[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            for (uint32_t b = halves[q]; b; b &= b - 1, --pairs)
+                item[at++] = (uint32_t)(4 * t + q) << 5 | (uint32_t)(__ffs((int)b) - 1);
+    }
+    __syncwarp();
+    const bool have = lane < allPairs;
+    const uint32_t it = have ? item[lane] : 0u;
+    const int half = (int)(it >> 5), word = half >> 1, bit = (int)(it & 31u);
+    const int jj = a.W == 1 ? word : word / a.W, wd = word - jj * a.W;
+    int u = -1, i = 0, h = 0;
+    if (have) {
+        const int off = __ldg(a.topK + (size_t)p * slots + jj) * 2 * a.m + (jj >= a.k ? a.m : 0) + wd * a.CT +
+                        (half & 1) * 32 + bit;
+        u = __ldg(a.slotMulti + off);
+        i = __ldg(a.topM + off);
+        h = np ? __ldg(a.slotHub + off) : 0;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, u >= 0 ? u : -2 - lane);
+    const bool first = have && lane == __ffs((int)same) - 1;
+    bool out1 = have && !first;
+    if (first) {
+        if (np <= kDdLists) {
+            for (int q = 0; q < np; ++q) {
+                const int l = sw.lists[q];
+                out1 |= (__ldg(a.kMask + (size_t)h * maskWords + (l >> 5)) >> (l & 31)) & 1u;
+            }
+        } else {
+            out1 = meets_list(a, listMask, i);
+        }
+        uint32_t* out = reinterpret_cast<uint32_t*>(a.accumulate ? a.newMasks : a.firstMasks);
+        atomicOr(out + row + half, 1u << bit);
+        if (a.accumulate) atomicOr(reinterpret_cast<uint32_t*>(a.firstMasks) + row + half, 1u << bit);
+    }
+    if (out1) atomicSub(a.inRaw + i, 1);
+    const int distinct = __popc(__ballot_sync(0xffffffffu, first));
+    __syncwarp();
+    return distinct;
+}
+
 // Persistent warps, each over points p = warp, warp + total, ...  A candidate
 // that no other list holds is a first occurrence as it stands.  The others are
 // gathered into a dense per-warp list (so the warp's instructions follow those
@@ -304,11 +366,20 @@ __global__ void __launch_bounds__(128, 8) k_core_dedupe(CoreArgs a, int seenWord
     for (int p = gw; p < a.n; p += nw) {
         const size_t row = (size_t)p * nHalves;
         // a point without a passing pair (common in a sweep round) only clears
-        // its first-occurrence words (this round's words when accumulating)
-        bool any = false;
-        for (int t = lane; t < nHalves; t += 32) any |= __ldg(mk32 + row + t) != 0u;
-        if (!__any_sync(0xffffffffu, any)) {
-            for (int t = lane; t < nHalves; t += 32) out[row + t] = 0u;
+        // its first-occurrence words (this round's words when accumulating);
+        // a row is an even number of words, 16 bytes at a time
+        int pairs = 0;  // this lane's passing pairs
+        const uint4* row4 = reinterpret_cast<const uint4*>(mk32 + row);
+        for (int t = lane; t < nHalves / 4; t += 32) {
+            const uint4 v = __ldg(row4 + t);
+            pairs += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+        }
+        const int allPairs = warp_sum(pairs);
+        if (allPairs <= 32) {
+            for (int t = lane; t < nHalves / 4; t += 32)
+                reinterpret_cast<uint4*>(out + row)[t] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (allPairs == 0) {
             if (lane == 0) a.aCount[p] = 0;
             continue;
         }
@@ -322,6 +393,11 @@ __global__ void __launch_bounds__(128, 8) k_core_dedupe(CoreArgs a, int seenWord
             mark_lists(a, listMask, h0, h0 + np, maskWords);
         }
         int distinct = 0;
+        if (allPairs <= 32) {
+            distinct = dedupe_sparse(a, sw, listMask, p, hub ? np : 0, pairs, allPairs);
+            if (lane == 0) a.aCount[p] = distinct;
+            continue;
+        }
         // pass s0 takes the candidates numbered [s0, s0 + span); the first one
         // takes those of a single list too
         for (int s0 = 0; s0 == 0 || s0 < multi; s0 += span) {
