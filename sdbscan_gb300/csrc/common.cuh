@@ -379,6 +379,8 @@ struct SngArgs {
     int32_t* nbIdx;
     float* nbDist;
     int32_t* err;          // set when a list would overflow its slots
+    float* colCopy;        // the packed tile's column copy (launch_sng_cols), or null: the scalar tile
+    const uint8_t* small;  // Chi2: DistArgs::small
     const uint64_t* heavy; // nct words: bit set for the columns drawn more than once (null: none)
     long long stallSpins;  // > 0: the stall test of k_sng_tc (sdb_set_debug_limits)
 };
@@ -421,7 +423,18 @@ struct SngBlockArgs {
     int32_t* hashId;         // -1 = empty
     float* hashDist;
     int32_t* err;            // set if a table overflows (cannot happen by construction)
+    float* colCopy;          // the packed tile's column copy (launch_sngb_cols), or null: the scalar tile
+    const uint8_t* small;    // Chi2: DistArgs::small
+    float* dists;            // sngOptics: blocks x S x 32 distances kept for the emitting pass, or null: computed again
 };
+// The packed tile of both rules (k_sng_pair.cu): the bytes of its copy of
+// `cols` columns (0: this distance has none), the copies, the kernels.
+size_t sng_pair_bytes(int dist, int64_t cols, int ld);
+int launch_sng_cols(const SngArgs& a, cudaStream_t st);
+int launch_sng_pair(const SngArgs& a, cudaStream_t st);
+int launch_sngb_cols(const SngBlockArgs& a, cudaStream_t st);
+int launch_sngb_pair(const SngBlockArgs& a, cudaStream_t st);
+int launch_sngb_insert(const SngBlockArgs& a, cudaStream_t st);
 int sng_block_rows();
 // pass words, degrees and core flags
 int launch_sngb_pass(const SngBlockArgs& a, int minPts, uint8_t* core, cudaStream_t st);

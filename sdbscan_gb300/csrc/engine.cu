@@ -44,9 +44,6 @@ namespace {
 // (launch_tile_order_list), and the key count of that order's counting sort.
 constexpr int kSuperChunk = 8;
 
-// Largest candidate copy of the packed distance tile (1M x 784 with D = 1024
-// and m = 50 takes 0.33 GB).
-constexpr size_t kMaxCandBytes = (size_t)8 << 30;
 constexpr int kMinCandMembers = 16;
 
 // Host input per upload segment.

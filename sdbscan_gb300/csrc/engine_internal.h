@@ -51,6 +51,10 @@ struct SweepSpec {
 //   [7] sng BF16 block failed (FP32 redoes it)   [8] a bounded wait of the plain distance kernel ran out
 constexpr int kErrSlots = 16;
 
+// Largest column copy of the packed distance tile (1M x 784 with D = 1024 and
+// m = 50 takes 0.33 GB).
+constexpr size_t kMaxCandBytes = (size_t)8 << 30;
+
 struct sdb_engine {
     int n = 0, d = 0, device = 0;
     sdb_params prm{};
@@ -129,6 +133,8 @@ struct sdb_engine {
     // labelsOut + i n when given) or sngOptics (one eps)
     sdb_status fit_sng(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
                        int32_t* labelsOut = nullptr, int32_t* nclOut = nullptr);
+    sdb_status fit_sng_once(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
+                            int32_t* labelsOut, int32_t* nclOut);
     // sngDbscan with independent samples per block of points (k_sng_blocks.cu)
     sdb_status fit_sng_blocks(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
                               int32_t* labelsOut, int32_t* nclOut);

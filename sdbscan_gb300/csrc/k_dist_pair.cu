@@ -3,16 +3,12 @@
 // for Cosine, L1, L2 and Chi2 with the packed FP32 tile of pair_tile.cuh.
 //
 // Tile = (list l, TM member rows, CT candidate columns), as in k_dist.cu; the
-// candidate rows come from a dimension-major copy that k_cand_tiles writes
+// candidate rows come from a dimension-major copy that k_col_tiles writes
 // once per fit (0.13 ms at 1M x 784, D = 1024, m = 50: every list's tile is
 // then one contiguous run per stage, read by about 50 row tiles).
 //
-// A list's last tile is rarely full (50K points, k = 5, D = 1024: 244 members
-// a list), so a tile runs with 2, 4, 6 or 8 rows per thread, whatever holds
-// its rows: the work follows the members to 48 rows instead of 192.
-//
 // Bound: the FP32 FMA pipe (72 % active at 1M x 784).
-#include "pair_tile.cuh"
+#include "pair_block.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -22,100 +18,40 @@ namespace {
 
 using namespace ptile;
 
-// The lists' candidate rows, dimension-major: column tile t = l nct + ct holds
-// ld runs of CTP floats, run k the k-th dimension of its CT candidates (zero
-// for columns past m); negated for L1 / L2.
-constexpr int kCtDims = 128;
-__global__ void __launch_bounds__(256) k_cand_tiles(DistArgs a, int CTP, int negate) {
-    __shared__ float tile[64][kCtDims + 1];
-    const int l = blockIdx.x / a.nct, ct = blockIdx.x % a.nct;
-    const int r = l % a.nproj, side = l / a.nproj;
-    const int32_t* cand = a.topM + (size_t)r * 2 * a.m + side * a.m;
-    const int k0 = blockIdx.y * kCtDims, kn = min(kCtDims, a.ld - k0);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int j = w; j < CTP; j += 8) {
-        const int c = ct * a.CT + j;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (j < a.CT && c < a.m && 4 * lane < kn) {
-            v = __ldg(reinterpret_cast<const float4*>(a.Xt + (size_t)__ldg(cand + c) * a.ld + k0) + lane);
-            if (negate) v = make_float4(-v.x, -v.y, -v.z, -v.w);
-        }
-        tile[j][4 * lane] = v.x;
-        tile[j][4 * lane + 1] = v.y;
-        tile[j][4 * lane + 2] = v.z;
-        tile[j][4 * lane + 3] = v.w;
+// The columns of list tile t = l nct + ct.
+struct ListCols {
+    const int32_t* topM;
+    int nproj, m, nct, CT;
+    __device__ int operator()(int64_t t, int j) const {
+        const int l = (int)(t / nct), c = (int)(t % nct) * CT + j;
+        return c < m ? __ldg(topM + (size_t)(l % nproj) * 2 * m + (l / nproj) * m + c) : -1;
     }
-    __syncthreads();
-    const int q4 = CTP / 4;
-    float4* out = reinterpret_cast<float4*>(a.cand + ((size_t)blockIdx.x * a.ld + k0) * CTP);
-    for (int e = threadIdx.x; e < kn * q4; e += blockDim.x) {
-        const int k = e / q4, q = e % q4;
-        out[e] = make_float4(tile[4 * q][k], tile[4 * q + 1][k], tile[4 * q + 2][k], tile[4 * q + 3][k]);
-    }
-}
+};
 
-template <class S> struct PairSmem {
-    float As[NST * S::TM * LDA];
-    float Bs[NST * KT * S::CTP];
-    int rowLoad[S::TM];   // point whose row is staged (the first member's past the tile's rows)
+// Writes the distances of a tile's pairs (sOPTICS and sweeps).
+template <class S, bool STORE> struct StoreDists {
+    const DistArgs& a;
+    const int* rowSlot;
+    int ct;
+    __device__ void operator()(int row, int p, int c, float d0, float d1, bool, bool) const {
+        if (!STORE) return;
+        const int left = a.m - ct * S::CT;  // columns of this tile
+        float* d = a.dists + ((size_t)p * 2 * a.k + rowSlot[row]) * a.m + ct * S::CT;
+        if (c < left) d[c] = d0;
+        if (c + 1 < left) d[c + 1] = d1;
+    }
+};
+
+template <class S> struct DistSmem {
+    PairSmem<S> t;
     int rowSlot[S::TM];
-    int colPoint[S::CT];  // -1 past m
-    int colCount[S::CT];
-    unsigned mask[2 * S::TM];
     int passTotal;
 };
 
-// Distances of a tile with up to RG * RM rows, and its pass bits, column
-// counts and (optionally) distances.
-template <int DIST, class S, int RM>
-__device__ __forceinline__ void pair_rows(const DistArgs& a, PairSmem<S>& sm, int rows, const float* cand, int ct) {
-    constexpr int kFinish = DIST == DIST_CHI2_ANY ? DIST_CHI2 : DIST;
-    u64 acc[RM][S::CN / 2];
-    pair_accumulate<DIST, S, RM>(a.Xt, a.ld, sm.rowLoad, cand, sm.As, sm.Bs, acc);
-    if (!S::active(threadIdx.x)) return;
-    int rg, tx;
-    S::coords(threadIdx.x, rg, tx);
-    int colPass[S::CN];
-#pragma unroll
-    for (int j = 0; j < S::CN; ++j) colPass[j] = 0;
-    const int left = a.m - ct * S::CT;  // columns of this tile
-#pragma unroll
-    for (int i = 0; i < RM; ++i) {
-        const int row = rg + S::RG * i;
-        if (row >= rows) continue;
-        const int p = sm.rowLoad[row];
-        float* dist = a.dists == nullptr ? nullptr
-                                         : a.dists + ((size_t)p * 2 * a.k + sm.rowSlot[row]) * a.m + ct * S::CT;
-        u64 bits = 0;
-#pragma unroll
-        for (int j = 0; j < S::CN / 2; ++j) {
-            const int c = S::column(tx, j);
-            float d0, d1;
-            unpack2(acc[i][j], d0, d1);
-            d0 = dtile::finish<kFinish>(d0);
-            d1 = dtile::finish<kFinish>(d1);
-            const int q0 = sm.colPoint[c], q1 = sm.colPoint[c + 1];
-            const bool p0 = d0 <= a.eps && q0 >= 0 && q0 != p, p1 = d1 <= a.eps && q1 >= 0 && q1 != p;
-            colPass[2 * j] += p0;
-            colPass[2 * j + 1] += p1;
-            bits |= (u64)((p0 ? 1u : 0u) | (p1 ? 2u : 0u)) << c;
-            if (dist != nullptr) {
-                if (c < left) dist[c] = d0;
-                if (c + 1 < left) dist[c + 1] = d1;
-            }
-        }
-        if ((unsigned)bits) atomicOr(&sm.mask[2 * row], (unsigned)bits);
-        if ((unsigned)(bits >> 32)) atomicOr(&sm.mask[2 * row + 1], (unsigned)(bits >> 32));
-    }
-#pragma unroll
-    for (int j = 0; j < S::CN; ++j)
-        if (colPass[j]) atomicAdd(&sm.colCount[S::column(tx, j >> 1) + (j & 1)], colPass[j]);
-}
-
-template <int DIST, class S>
+template <int DIST, class S, bool STORE>
 __global__ void __launch_bounds__(kThreads, 3) k_dist_pair(DistArgs a) {
     extern __shared__ __align__(16) unsigned char raw[];
-    PairSmem<S>& sm = *reinterpret_cast<PairSmem<S>*>(raw);
+    DistSmem<S>& sm = *reinterpret_cast<DistSmem<S>*>(raw);
     const int tid = threadIdx.x;
     if ((int64_t)blockIdx.x >= *a.tileTotal) return;
     const int64_t t = tile_at(a.tilePerm, blockIdx.x);
@@ -124,63 +60,42 @@ __global__ void __launch_bounds__(kThreads, 3) k_dist_pair(DistArgs a) {
     const int mt = (int)(ti / a.nct), ct = (int)(ti % a.nct);
     const int64_t mbeg = a.listOff[l] + (int64_t)mt * S::TM;
     const int rows = (int)min((int64_t)S::TM, a.listOff[l + 1] - mbeg);
-    const int r = l % a.nproj, side = l / a.nproj;
-    const int32_t* list = a.topM + (size_t)r * 2 * a.m + side * a.m;
+    const ListCols cols{a.topM, a.nproj, a.m, a.nct, S::CT};
     for (int i = tid; i < S::TM; i += kThreads) {
         const int2 mb = a.members[mbeg + (i < rows ? i : 0)];
-        sm.rowLoad[i] = mb.x;
+        sm.t.rowLoad[i] = mb.x;
         sm.rowSlot[i] = mb.y;
-        sm.mask[2 * i] = 0;
-        sm.mask[2 * i + 1] = 0;
     }
-    for (int j = tid; j < S::CT; j += kThreads) {
-        const int c = ct * S::CT + j;
-        sm.colPoint[j] = c < a.m ? list[c] : -1;
-        sm.colCount[j] = 0;
-    }
+    for (int j = tid; j < S::CT; j += kThreads) sm.t.colPoint[j] = cols((int64_t)l * a.nct + ct, j);
     if (tid == 0) sm.passTotal = 0;
-    bool small = false;  // Chi2: a row or a candidate of the tile has an entry below kChi2Small
-    if (DIST == DIST_CHI2) {
-        for (int i = tid; i < rows; i += kThreads) small |= a.small[sm.rowLoad[i]] != 0;
-        for (int j = tid; j < S::CT; j += kThreads) small |= sm.colPoint[j] >= 0 && a.small[sm.colPoint[j]] != 0;
-    }
-    small = __syncthreads_or(small);
-
-    const float* cand = a.cand + ((size_t)l * a.nct + ct) * a.ld * S::CTP;
-    const int need = (rows + S::RG - 1) / S::RG;  // rows per thread
-    if (DIST == DIST_CHI2 && small) pair_rows<DIST_CHI2_ANY, S, S::RMAX>(a, sm, rows, cand, ct);
-    else if (need <= 2) pair_rows<DIST, S, 2>(a, sm, rows, cand, ct);
-    else if (need <= 4) pair_rows<DIST, S, 4>(a, sm, rows, cand, ct);
-    else if (S::RMAX == 6 || need <= 6) pair_rows<DIST, S, 6>(a, sm, rows, cand, ct);
-    else pair_rows<DIST, S, S::RMAX>(a, sm, rows, cand, ct);
-    __syncthreads();
+    pair_tile<DIST, S>(PairTile{a.Xt, a.ld, a.eps, a.cand + ((size_t)l * a.nct + ct) * a.ld * S::CTP, rows}, sm.t,
+                       a.small, StoreDists<S, STORE>{a, sm.rowSlot, ct});
 
     int pass = 0;
     for (int row = tid; row < rows; row += kThreads) {
-        const u64 w = ((u64)sm.mask[2 * row + 1] << 32) | sm.mask[2 * row];
-        a.masks[((size_t)sm.rowLoad[row] * 2 * a.k + sm.rowSlot[row]) * a.W + ct] = w;
+        const u64 w = ((u64)sm.t.mask[2 * row + 1] << 32) | sm.t.mask[2 * row];
+        a.masks[((size_t)sm.t.rowLoad[row] * 2 * a.k + sm.rowSlot[row]) * a.W + ct] = w;
         pass += __popcll(w);
     }
     for (int j = tid; j < S::CT; j += kThreads)
-        if (sm.colCount[j]) atomicAdd(a.inRaw + sm.colPoint[j], sm.colCount[j]);
+        if (sm.t.colCount[j]) atomicAdd(a.inRaw + sm.t.colPoint[j], sm.t.colCount[j]);
     pass = warp_sum(pass);
     if ((tid & 31) == 0 && pass) atomicAdd(&sm.passTotal, pass);
     __syncthreads();
     if (tid == 0 && sm.passTotal) atomicAdd(a.pairs, (unsigned long long)sm.passTotal);
 }
 
-using Shape32 = PairShape<4, 8, 6>;
-using Shape40 = PairShape<5, 8, 8>;
-using Shape50 = PairShape<5, 10, 8>;
-using Shape64 = PairShape<8, 8, 8>;
-
-template <int DIST, class S> int launch_pair_t(const DistArgs& a, cudaStream_t st) {
-    const size_t sm = sizeof(PairSmem<S>);
-    if (cudaFuncSetAttribute(k_dist_pair<DIST, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
+template <int DIST, class S, bool STORE> int launch_pair_s(const DistArgs& a, cudaStream_t st) {
+    const size_t sm = sizeof(DistSmem<S>);
+    if (cudaFuncSetAttribute(k_dist_pair<DIST, S, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
         cudaSuccess)
         return -1;
-    k_dist_pair<DIST, S><<<(unsigned)a.nTiles, kThreads, sm, st>>>(a);
+    k_dist_pair<DIST, S, STORE><<<(unsigned)a.nTiles, kThreads, sm, st>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+
+template <int DIST, class S> int launch_pair_t(const DistArgs& a, cudaStream_t st) {
+    return a.dists != nullptr ? launch_pair_s<DIST, S, true>(a, st) : launch_pair_s<DIST, S, false>(a, st);
 }
 
 template <int DIST> int launch_pair_d(const DistArgs& a, cudaStream_t st) {
@@ -222,9 +137,8 @@ size_t pair_cand_bytes(int cols, int nproj, int m, int ld) {
 }
 
 int launch_cand_tiles(const DistArgs& a, cudaStream_t st) {
-    const dim3 grid((unsigned)(2 * a.nproj * a.nct), (unsigned)((a.ld + kCtDims - 1) / kCtDims));
-    k_cand_tiles<<<grid, 256, 0, st>>>(a, pair_tile_ctp(a.CT), a.dist == DIST_COSINE ? 0 : 1);
-    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+    return launch_col_tiles(a.Xt, a.ld, a.dist, ListCols{a.topM, a.nproj, a.m, a.nct, a.CT},
+                            (int64_t)2 * a.nproj * a.nct, a.CT, pair_tile_ctp(a.CT), a.cand, st);
 }
 
 int launch_dist_pair(const DistArgs& a, cudaStream_t st) {

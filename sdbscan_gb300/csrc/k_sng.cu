@@ -9,8 +9,9 @@
 // their multiplicities) and, for each sampled point, the few extra draws that
 // replace its own occurrences.  The GPU work is then a dense block: every
 // point (row) against every distinct sampled point (column), computed with
-// the FP32 distance tile of the candidate stage (same rounding sequence as
-// the CPU path), plus a short list of extra pairs.
+// the packed FP32 distance tile (k_sng_pair.cu) or, for JS, sngOptics and a
+// column copy that does not fit in memory, the scalar one here (the same
+// rounding sequence as the CPU path), plus a short list of extra pairs.
 //
 // Per pass (p, q), p != q, dist <= eps:
 //  - sngDbscan, sampled (:446-464): p's list gets q and q's list gets p once
@@ -337,7 +338,9 @@ int grid_for(int64_t work, int threads) {
 
 }  // namespace
 
-int launch_sng_block(const SngArgs& a, cudaStream_t st) { return launch_block<false>(a, st); }
+int launch_sng_block(const SngArgs& a, cudaStream_t st) {
+    return a.colCopy != nullptr ? launch_sng_pair(a, st) : launch_block<false>(a, st);
+}
 int launch_sng_emit(const SngArgs& a, cudaStream_t st) { return launch_block<true>(a, st); }
 
 int launch_sng_extras(const SngArgs& a, cudaStream_t st) {

@@ -17,10 +17,12 @@
 // word per (block, draw) over the block's points; the union-find and border
 // passes walk the words.
 //
-// The distance tile is the candidate stage's FP32 tile (dist_tile.cuh): every
+// The distance tile is the packed FP32 tile (k_sng_pair.cu) or, for JS and
+// where its column copy does not fit in memory, the scalar one here: every
 // distance is the CPU path's bits, so the result equals the oracle's
 // restatement of the same rule (orc_fit_sngdbscan_blocks).
 #include "dist_tile.cuh"
+#include "sng_draws.cuh"
 #include "uf.cuh"
 
 #include <algorithm>
@@ -31,45 +33,11 @@ namespace {
 
 using namespace dtile;
 
-constexpr int BR = 32;                       // points per sampled block
+constexpr int BR = kSngBlockRows;            // points per sampled block
 constexpr int BTX = 8, BCN = 4, BNT = 16 * BTX;  // 128 draws x 32 points on 128 threads
-
-__device__ __forceinline__ uint64_t splitmix64(uint64_t z) {
-    z += 0x9E3779B97F4A7C15ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
-
-__device__ __forceinline__ int block_draw(uint64_t key, int64_t S, int64_t b, int64_t j, int n) {
-    const uint64_t z = splitmix64(key + (uint64_t)(b * S + j));
-    return (int)(((z >> 32) * (uint64_t)n) >> 32);
-}
 
 size_t tile_smem() {
     return sizeof(float) * (STAGES * (TM + BTX * BCN) * LDS) + sizeof(int) * (TM + BTX * BCN);
-}
-
-// sngOptics: q into p's open-addressing table of distinct neighbours (ids,
-// -1 = empty, with the pair's distance), linear probing from a
-// multiplicative hash.
-__device__ __forceinline__ void hash_insert(const SngBlockArgs& a, int p, int q, float dist) {
-    const int64_t o = a.hashOff[p];
-    const int cap = (int)(a.hashOff[p + 1] - o);
-    if (cap == 0) {
-        atomicExch(a.err, 1);
-        return;
-    }
-    uint32_t h = ((uint32_t)q * 0x9E3779B1u) & (uint32_t)(cap - 1);
-    for (int probe = 0; probe < cap; ++probe, h = (h + 1) & (uint32_t)(cap - 1)) {
-        const int old = atomicCAS(a.hashId + o + h, -1, q);
-        if (old == -1) {  // first occurrence of q in p's list
-            a.hashDist[o + h] = dist;
-            return;
-        }
-        if (old == q) return;  // a repeat: dist(p, q) is the same value every time
-    }
-    atomicExch(a.err, 1);  // full table (cannot happen: cap >= 2 x the entries)
 }
 
 // One tile (block b, draws dt * 128 ..) per CTA.  Tiles of a block are
@@ -260,6 +228,8 @@ template <int DIST, bool EMIT> int launch_tile_t(const SngBlockArgs& a, cudaStre
 }
 
 template <bool EMIT> int launch_tiles(const SngBlockArgs& a, cudaStream_t st) {
+    if (!EMIT && a.colCopy != nullptr) return launch_sngb_pair(a, st);
+    if (EMIT && a.dists != nullptr) return launch_sngb_insert(a, st);
     switch (a.dist) {
         case DIST_COSINE: return launch_tile_t<DIST_COSINE, EMIT>(a, st);
         case DIST_L1: return launch_tile_t<DIST_L1, EMIT>(a, st);

@@ -100,6 +100,20 @@ const char* dist_label(int d) {
 
 sdb_status sdb_engine::fit_sng(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts,
                                bool optics, int32_t* labelsOut, int32_t* nclOut) {
+    sdb_status s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut);
+    // out of memory with the packed tile's column copy: once more without it
+    if (s == SDB_ERR_NOMEM && candT.ptr != nullptr) {
+        cudaStreamSynchronize(stream);
+        release(candT);
+        release(dists);
+        noCandCopy = true;
+        s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut);
+    }
+    return s;
+}
+
+sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts,
+                                    bool optics, int32_t* labelsOut, int32_t* nclOut) {
     if (!paramsSet && !sngParamsSet) return fail(SDB_ERR_STATE, "set_sngParams must be called before a fit");
     if (X == nullptr) return fail(SDB_ERR_ARG, "X is null");
     if (epsList == nullptr || nEps < 1 || (optics && nEps != 1)) return fail(SDB_ERR_ARG, "invalid eps list");
@@ -141,6 +155,12 @@ sdb_status sdb_engine::fit_sng(const float* X, bool xOnDevice, const float* epsL
           ensure(sngExtraPass, std::max(nExtra, 1)) && ensure(rowDeg, sizeof(int32_t) * n) &&
           ensure(colCnt, sizeof(int32_t) * std::max(nU, 1)) && ensure(degree, sizeof(int32_t) * n) &&
           ensure(core, n) && ensure(scanTmp, sizeof(int64_t) * scan_tmp_elems((size_t)n + 1));
+    // the packed tile for the FP32 block of sngDbscan (the screened one needs it
+    // only if the screening fails)
+    const bool screen = !optics && p.precision == SDB_PREC_BF16 && p.distance == SDB_COSINE && nU > 0;
+    const size_t copyBytes = optics || screen ? 0 : sng_pair_bytes(p.distance, nU, ld);
+    const bool packed = copyBytes > 0 && !noCandCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
+                        (p.distance != SDB_CHI2 || ensure(smallEntry, n));
     if (!optics)
         ok &= ensure(sngMask, sizeof(uint64_t) * std::max<size_t>(1, (size_t)nct * n)) &&
               ensure(parent, sizeof(int32_t) * n) && ensure(border, sizeof(int32_t) * n) &&
@@ -183,6 +203,7 @@ sdb_status sdb_engine::fit_sng(const float* X, bool xOnDevice, const float* epsL
     pa.dist = p.distance;
     pa.scale = f32(scale);
     pa.err = i32(errFlags);
+    if (packed && p.distance == SDB_CHI2) pa.small = static_cast<uint8_t*>(smallEntry.ptr);
     L_(launch_transform(pa, st));
     SDB_CK(cudaEventRecord(ev[2], st));
     SDB_CK(cudaEventRecord(ev[3], st));
@@ -215,9 +236,13 @@ sdb_status sdb_engine::fit_sng(const float* X, bool xOnDevice, const float* epsL
     sa.err = i32(errFlags) + 6;
     sa.stallSpins = dbgStallSpins;
     L_(launch_sng_col_of(sa, i32(sngColOf), st));
+    if (packed) {
+        sa.colCopy = f32(candT);
+        sa.small = static_cast<const uint8_t*>(smallEntry.ptr);
+        L_(launch_sng_cols(sa, st));
+    }
     // BF16 screening of the block (Cosine sngDbscan): BF16 copies of every
     // row and of the sampled rows, a queue for the pairs near eps
-    const bool screen = !optics && p.precision == SDB_PREC_BF16 && p.distance == SDB_COSINE && nU > 0;
     const int ldb = (d + 63) / 64 * 64;
     int64_t qcap = 0;
     std::vector<uint64_t> heavy;  // per 64-column word: the columns drawn more than once
@@ -373,6 +398,12 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
           ensure(labels, sizeof(int32_t) * n) && ensure(nClusters, sizeof(int32_t) * 4) &&
           ensure(scanTmp, sizeof(int64_t) * scan_tmp_elems((size_t)n + 1)) &&
           ensure(sngWords, sizeof(uint32_t) * std::max<size_t>(1, (size_t)nb * (size_t)std::max<int64_t>(S, 0)));
+    const size_t copyBytes = S > 0 ? sng_pair_bytes(p.distance, n, ld) : 0;
+    const bool packed = copyBytes > 0 && !noCandCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
+                        (p.distance != SDB_CHI2 || ensure(smallEntry, n));
+    // sngOptics keeps the pass's distances for its emitting pass
+    const size_t distBytes = sizeof(float) * (size_t)nb * BR * (size_t)std::max<int64_t>(S, 0);
+    const bool keepDists = optics && packed && distBytes <= kMaxCandBytes && ensure(dists, distBytes);
     if (optics)
         ok &= ensure(nbOff, sizeof(int64_t) * (n + 1)) && ensure(coreDist, sizeof(float) * n) &&
               ensure(hashOffB, sizeof(int64_t) * (n + 1));
@@ -408,6 +439,7 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
     pa.dist = p.distance;
     pa.scale = f32(scale);
     pa.err = i32(errFlags);
+    if (packed && p.distance == SDB_CHI2) pa.small = static_cast<uint8_t*>(smallEntry.ptr);
     L_(launch_transform(pa, st));
     SDB_CK(cudaEventRecord(ev[2], st));
     SDB_CK(cudaEventRecord(ev[3], st));
@@ -429,6 +461,12 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
     ba.degree = i32(degree);
     ba.pairs = ctr + 3;
     ba.err = i32(errFlags) + 6;
+    if (packed) {
+        ba.colCopy = f32(candT);
+        ba.small = static_cast<const uint8_t*>(smallEntry.ptr);
+        if (keepDists) ba.dists = f32(dists);
+        L_(launch_sngb_cols(ba, st));
+    }
     if (optics) {
         // passes with repeats -> table sizes -> the emitting pass into the
         // tables -> distinct lists, core flags and core distances -> ordering
