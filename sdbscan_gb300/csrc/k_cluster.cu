@@ -47,20 +47,18 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
     return true;
 }
 
-// Before the tile pass: rounds of hooking without unites.  A core point (in an
-// eps sweep one that became core this round) looks at two passing candidates
-// of two of its lists and hooks its root under the smallest root it sees, by a
-// plain atomicMin: parents only move down, so the forest stays a forest, and
-// where one root is hooked twice the tile pass, which sees every edge, restores
-// the other link.  With every point a set of its own the tile pass would send
-// some twenty unites per point at the same few roots, all at once; after the
-// rounds it finds mostly equal roots (50K x 128: union 379 us without, 100 plus
-// 45 for the rounds; 1M x 784: 1827 and 955 + 292).
+// Before the tile pass: rounds of hooking (RootSpan).  A core point (in an eps
+// sweep one that became core this round) looks at two passing candidates of two
+// of its lists and hooks the roots it sees; the tile pass sees every edge and
+// restores a link that two hooks of one root lost.  With every point a set of
+// its own the tile pass would send some twenty unites per point at the same few
+// roots, all at once; after the rounds it finds almost nothing but equal roots
+// (50K x 128: union 379 us without, 35 plus 45 for the rounds; 1M x 784: 1827
+// and 613 + 263; hooking only the own root left 100 and 955).
 __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p] || (a.carry && a.coreEps[p] != a.round)) return;
-    const int r = load_parent(a.parent, p);
-    int best = r;
+    RootSpan span(load_parent(a.parent, p));
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int j = (slot0 + t) % (2 * a.k);
@@ -70,10 +68,10 @@ __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
         const int32_t* cand = a.topM + (size_t)__ldg(a.topK + at) * 2 * a.m + (j >= a.k ? a.m : 0);
         for (int c = 0; c < 2 && bits; ++c, bits &= bits - 1) {
             const int q = __ldg(cand + __ffsll((long long)bits) - 1);
-            if (a.core[q]) best = min(best, load_parent(a.parent, q));
+            if (a.core[q]) span.see(load_parent(a.parent, q));
         }
     }
-    if (best < r) atomicMin(a.parent + r, best);
+    span.hook(a.parent);
 }
 
 // The tile's candidates of one root, as a bit set.
@@ -229,9 +227,9 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st) {
     const int g = (a.n + 255) / 256;
     k_init<<<g, 256, 0, st>>>(a.parent, a.border, a.n, a.carry && a.round > 0);
     ++launches;
-    // three rounds over two lists, two candidates of each (33K x 333 cluster
-    // stage: 0.49 ms with one round over one candidate, 0.35 with two rounds,
-    // 0.26 with three); a sweep's later rounds have few new core points
+    // three rounds over two lists, two candidates of each (33K x 333, 10 clusters:
+    // one round over one candidate leaves the stage at 0.49 ms, three at 0.16); a
+    // sweep's later rounds have few new core points
     const int rounds = !a.carry ? 3 : a.round == 0 ? 2 : 1;
     for (int t = 0; t < rounds; ++t) {
         k_hook<<<g, 256, 0, st>>>(a, 2 * t);

@@ -18,20 +18,18 @@
 namespace sdb {
 namespace {
 
-// A core point's root under the smallest root among four of its core
-// neighbours (plain atomicMin, as k_hook of the cluster stage; the union pass
-// sees every edge).
+// A core point hooks its root and those of four of its core neighbours
+// (RootSpan; the union pass sees every edge).
 __global__ void k_csr_hook(CsrArgs a, int from) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p]) return;
     const int64_t e0 = a.off[p], len = a.off[p + 1] - e0;
-    const int r = load_parent(a.parent, p);
-    int best = r;
+    RootSpan span(load_parent(a.parent, p));
     for (int t = from; t < from + 4 && t < len; ++t) {
         const int q = __ldg(a.idx + e0 + t);
-        if (a.core[q]) best = min(best, load_parent(a.parent, q));
+        if (a.core[q]) span.see(load_parent(a.parent, q));
     }
-    if (best < r) atomicMin(a.parent + r, best);
+    span.hook(a.parent);
 }
 
 __global__ void k_csr_compress(CsrArgs a) {

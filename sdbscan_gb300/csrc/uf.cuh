@@ -35,4 +35,23 @@ static __device__ void unite(int32_t* parent, int a, int b) {
     }
 }
 
+// Hooking without unites: a point that saw the roots r (its own) and others of
+// its component hooks the largest of them and its own under the smallest, by
+// plain atomicMin.  Parents only move down, so the forest stays a forest; where
+// one root is hooked twice one link is lost, so a pass over every edge has to
+// follow.  (The largest as well: a root below every root it sees would
+// otherwise wait for the unites.)
+struct RootSpan {
+    int own, lo, hi;
+    __device__ explicit RootSpan(int r) : own(r), lo(r), hi(r) {}
+    __device__ void see(int r) {
+        lo = min(lo, r);
+        hi = max(hi, r);
+    }
+    __device__ void hook(int32_t* parent) const {
+        if (lo < own) atomicMin(parent + own, lo);
+        if (lo < hi && hi != own) atomicMin(parent + hi, lo);
+    }
+};
+
 }  // namespace sdb
