@@ -151,6 +151,8 @@ int launch_topm_select(const TopMArgs& a, cudaStream_t st);
 // scan_tmp_elems(n) entries.
 size_t scan_tmp_elems(size_t n);
 int launch_scan_i64(const int64_t* in, int64_t* out, size_t n, int64_t* tmp, cudaStream_t st);
+// The same of n int32 values; out gets n + 1 entries (the total last).
+int launch_scan_i32(const int32_t* in, size_t n, int64_t* out, int64_t* tmp, cudaStream_t st);
 
 struct IndexArgs {
     const int32_t* topK;  // n x 2k
@@ -179,7 +181,9 @@ struct IndexArgs {
 // Members of every list ordered by point chunk (CTA per chunk).
 int launch_index_count(const IndexArgs& a, cudaStream_t st);
 int launch_index_scatter(const IndexArgs& a, cudaStream_t st);
-// tilePerm: the tiles sorted by the chunk of their first member.
+// tileOff: the lists' tile counts, scanned.
+int launch_tile_offsets(const IndexArgs& a, cudaStream_t st);
+// tileList, and tilePerm: the tiles sorted by the chunk of their first member.
 int launch_tile_order(const IndexArgs& a, cudaStream_t st);
 // tilePerm for the tensor-core distance kernel: tiles by (super-chunk of
 // superChunk point chunks, list); keys: total tiles, keyOff:
@@ -189,7 +193,6 @@ int launch_tile_order_list(const IndexArgs& a, int superChunk, int32_t* keys, in
                            cudaStream_t st);
 // Tile id of the b-th launched tile (identity without a permutation).
 __device__ __forceinline__ int64_t tile_at(const int32_t* perm, int64_t b) { return perm != nullptr ? perm[b] : b; }
-int launch_tiles(const IndexArgs& a, int64_t total_tiles, cudaStream_t st);
 int launch_hubs_count(const IndexArgs& a, cudaStream_t st);
 int launch_hubs_scatter(const IndexArgs& a, cudaStream_t st);
 
@@ -322,7 +325,7 @@ struct ClusterArgs {
     const uint8_t* core;
     int32_t* parent;
     int32_t* border;
-    int64_t* rootFlag;    // n + 1, scanned into cluster ids
+    int64_t* rootFlag;    // n + 1: scan of the root flags (cluster ids)
     int64_t* scanTmp;
     int32_t* labels;
     int32_t* nClusters;   // device scalar
@@ -332,6 +335,13 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st);
 // = p and border[p] = INT_MAX; parents of core points set to their roots;
 // cluster ids and labels from core, parent and border (uses n, core, parent,
 // border, rootFlag, scanTmp, labels, nClusters).
+// Between hooking rounds: the same compression from this many points on.  Below
+// it the rounds' own path halving is as good and a launch cheaper (50K points:
+// 5 us a round); above it the paths the next round walks cost more (200K x 784,
+// unseeded sngDbscan: cluster stage 0.94 ms without, 0.63 with; 1M x 784
+// 1.5 and 1.1).
+constexpr int kCompressRounds = 100000;
+int launch_uf_compress_round(int n, const uint8_t* core, int32_t* parent, cudaStream_t st);
 int launch_uf_init(int32_t* parent, int32_t* border, int n, cudaStream_t st);
 int launch_uf_compress(const ClusterArgs& a, cudaStream_t st);
 int launch_cluster_labels(const ClusterArgs& a, cudaStream_t st);

@@ -29,8 +29,6 @@
 #include "engine_internal.h"
 
 namespace sdb {
-int launch_tile_offsets(const IndexArgs& a, cudaStream_t st);
-int launch_i32_to_i64(const int32_t* in, int64_t* out, int n, cudaStream_t st);
 int dist_tile_rows();
 int dist_tile_cols();
 int launch_pad_copy(const float* X, int n, int d, float* Xt, int ld, cudaStream_t st);
@@ -40,9 +38,10 @@ using namespace sdb;
 
 namespace {
 
-// Point chunks per super-chunk of the tensor-core distance kernel's tile order
+// Points per chunk of the index kernels, at most; chunks of that size per
+// super-chunk of the tensor-core distance kernel's tile order
 // (launch_tile_order_list), and the key count of that order's counting sort.
-constexpr int kSuperChunk = 8;
+constexpr int kChunkPts = 4096, kSuperChunk = 8;
 
 constexpr int kMinCandMembers = 16;
 
@@ -50,7 +49,7 @@ constexpr int kMinCandMembers = 16;
 constexpr size_t kSegBytes = (size_t)256 << 20;
 
 size_t kTcKeys(int n, int L) {
-    const int nChunks = (n + 4095) / 4096;
+    const int nChunks = (n + kChunkPts - 1) / kChunkPts;
     return (size_t)((nChunks + kSuperChunk - 1) / kSuperChunk) * L + 1;
 }
 
@@ -296,7 +295,13 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
           ensure(errFlags, sizeof(int32_t) * kErrSlots) && ensure(counters, sizeof(unsigned long long) * 8) &&
           ensure(signs, sizeof(uint32_t) * hostSigns.size()) &&
           ensure(compCosh, sizeof(double) * std::max<size_t>(1, hostCosh.size()));
-    const int chunkPts = 4096, nChunks = (n + chunkPts - 1) / chunkPts;
+    // points per CTA of the index kernels: 4096, fewer where those would leave
+    // SMs without one (50K points: 13 CTAs, count and scatter 63 us; 196 of 256
+    // points, 17)
+    int chunkPts = kChunkPts;
+    while (chunkPts > 256 && (int64_t)chunkPts * sm_count() > n) chunkPts >>= 1;
+    const int nChunks = (n + chunkPts - 1) / chunkPts;
+    const int superChunk = kSuperChunk * (kChunkPts / chunkPts);  // the same points whatever a chunk holds
     ok &= ensure(chunkOff, sizeof(int32_t) * (size_t)L * nChunks) && ensure(tileKey, sizeof(int32_t) * maxTiles) &&
           ensure(keyOff, sizeof(int64_t) * ((size_t)nChunks + 1)) && ensure(tilePerm, sizeof(int32_t) * maxTiles);
     const int maskWords = (L + 31) / 32;
@@ -486,16 +491,13 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     ia.maxTiles = maxTiles;
     SDB_CK(cudaMemsetAsync(listCount.ptr, 0, sizeof(int64_t) * (L + 1), st));
     SDB_CK(cudaMemsetAsync(hubCount.ptr, 0, sizeof(int32_t) * n, st));
-    SDB_CK(cudaMemsetAsync(hubOff.ptr, 0, sizeof(int64_t) * (n + 1), st));
     L_(launch_index_count(ia, st));
     L_(launch_scan_i64(i64(listCount), i64(listOff), (size_t)L + 1, i64(scanTmp), st));
     L_(launch_index_scatter(ia, st));
     L_(launch_tile_offsets(ia, st));
-    L_(launch_tiles(ia, 0, st));
     L_(launch_tile_order(ia, st));
     L_(launch_hubs_count(ia, st));
-    L_(launch_i32_to_i64(i32(hubCount), i64(hubOff), n, st));
-    L_(launch_scan_i64(i64(hubOff), i64(hubOff), (size_t)n + 1, i64(scanTmp), st));
+    L_(launch_scan_i32(i32(hubCount), n, i64(hubOff), i64(scanTmp), st));
     SDB_CK(cudaMemsetAsync(hubCount.ptr, 0, sizeof(int32_t) * n, st));
     L_(launch_hubs_scatter(ia, st));
     if (optics) L_(launch_slot_sigs(i32(topM), D, m, i64(hubOff), i32(hubLists), sig.ptr, st));
@@ -561,11 +563,11 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
         }
         // the tensor-core kernel takes the tiles by (super-chunk, list): the
         // rows of 8 point chunks stay in L2 while every list passes over them
-        const size_t nKeys = tile_order_list_keys(ia, kSuperChunk);
+        const size_t nKeys = tile_order_list_keys(ia, superChunk);
         if (!ensure(tileKeyTc, sizeof(int32_t) * (size_t)maxTiles) || !ensure(keyOffTc, sizeof(int64_t) * nKeys) ||
             !ensure(tilePermTc, sizeof(int32_t) * (size_t)maxTiles))
             return SDB_ERR_NOMEM;
-        L_(launch_tile_order_list(ia, kSuperChunk, i32(tileKeyTc), i64(keyOffTc), i32(tilePermTc), st));
+        L_(launch_tile_order_list(ia, superChunk, i32(tileKeyTc), i64(keyOffTc), i32(tilePermTc), st));
         DistArgs dtc = da;
         dtc.tilePerm = i32(tilePermTc);
         L_(launch_dist_tc(dtc, Xb.ptr, ldb, Cb.ptr, static_cast<uint64_t*>(queue.ptr), qcap, ctr + 4,

@@ -11,6 +11,7 @@
 //    there is no cluster (:619, :633).
 // Union-find hooks the larger root under the smaller one, so each root is
 // its component's minimum index and ids follow from a prefix sum over roots.
+#include "scan.cuh"
 #include "uf.cuh"
 
 #include <climits>
@@ -58,7 +59,7 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
 __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p] || (a.carry && a.coreEps[p] != a.round)) return;
-    RootSpan span(load_parent(a.parent, p));
+    RootSpan span(round_root(a.parent, p, a.n));
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int j = (slot0 + t) % (2 * a.k);
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
         const int32_t* cand = a.topM + (size_t)__ldg(a.topK + at) * 2 * a.m + (j >= a.k ? a.m : 0);
         for (int c = 0; c < 2 && bits; ++c, bits &= bits - 1) {
             const int q = __ldg(cand + __ffsll((long long)bits) - 1);
-            if (a.core[q]) span.see(load_parent(a.parent, q));
+            if (a.core[q]) span.see(round_root(a.parent, q, a.n));
         }
     }
     span.hook(a.parent);
@@ -201,22 +202,45 @@ __global__ void __launch_bounds__(256) k_border_tiles(ClusterArgs a) {
     if (q >= 0 && cbest[threadIdx.x] != INT_MAX) atomicMin(a.border + q, cbest[threadIdx.x]);
 }
 
-__global__ void k_root_flags(ClusterArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > a.n) return;
-    a.rootFlag[p] = (p < a.n && a.core[p] && a.parent[p] == p) ? 1 : 0;
-}
+// 1 for a root (a core point that is its own parent).
+struct RootFlags {
+    const uint8_t* core;
+    const int32_t* parent;
+    int n;
+    __device__ int64_t operator()(size_t p) const { return p < (size_t)n && core[p] && parent[p] == (int)p ? 1 : 0; }
+};
 
-__global__ void k_labels(ClusterArgs a) {
+// nb > 0: rootFlag holds sums within tiles; sums the tiles' totals, which the
+// block scans for itself.
+__global__ void __launch_bounds__(scan::kThreads) k_labels(ClusterArgs a, const int64_t* __restrict__ sums, int nb) {
+    __shared__ int64_t off[scan::kSumsInSmem];
+    if (nb > 0) {
+        constexpr int kPer = scan::kSumsInSmem / scan::kThreads;
+        int64_t v[kPer], s = 0, total;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int t = (int)threadIdx.x * kPer + i;
+            v[i] = t < nb ? __ldg(sums + t) : 0;
+            s += v[i];
+        }
+        int64_t ex = scan::block_exclusive<scan::kThreads>(s, &total);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            off[threadIdx.x * kPer + i] = ex;
+            ex += v[i];
+        }
+        __syncthreads();
+    }
+    auto id = [&](int root) { return (int)(a.rootFlag[root] + (nb > 0 ? off[root / scan::kTile] : 0)); };
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p == 0) {
-        const int c = (int)a.rootFlag[a.n];
+        const int c = id(a.n);
         *a.nClusters = c >= 1 ? c + 1 : 2;
     }
     if (p >= a.n) return;
     int lab = -1;
-    if (a.core[p]) lab = (int)a.rootFlag[a.parent[p]];
-    else if (a.border[p] != INT_MAX) lab = (int)a.rootFlag[a.border[p]];
+    if (a.core[p]) lab = id(a.parent[p]);
+    else if (a.border[p] != INT_MAX) lab = id(a.border[p]);
     a.labels[p] = lab;
 }
 
@@ -231,10 +255,11 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st) {
     // one round over one candidate leaves the stage at 0.49 ms, three at 0.16); a
     // sweep's later rounds have few new core points
     const int rounds = !a.carry ? 3 : a.round == 0 ? 2 : 1;
-    for (int t = 0; t < rounds; ++t) {
+    for (int t = 0; t < rounds; ++t, ++launches) {
         k_hook<<<g, 256, 0, st>>>(a, 2 * t);
-        k_compress<<<g, 256, 0, st>>>(a);
-        launches += 2;
+        const int r = launch_uf_compress_round(a.n, a.core, a.parent, st);
+        if (r < 0) return -1;
+        launches += r;
     }
     k_union_tiles<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     ++launches;
@@ -242,14 +267,8 @@ int launch_cluster(const ClusterArgs& a, cudaStream_t st) {
     ++launches;
     k_border_tiles<<<(unsigned)a.nTiles, a.TM, 0, st>>>(a);
     ++launches;
-    k_root_flags<<<(a.n + 1 + 255) / 256, 256, 0, st>>>(a);
-    ++launches;
-    int r = launch_scan_i64(a.rootFlag, a.rootFlag, (size_t)a.n + 1, a.scanTmp, st);
-    if (r < 0) return -1;
-    launches += r;
-    k_labels<<<g, 256, 0, st>>>(a);
-    ++launches;
-    return cudaPeekAtLastError() == cudaSuccess ? launches : -1;
+    const int r = launch_cluster_labels(a, st);
+    return r < 0 ? -1 : launches + r;
 }
 
 // The union-find steps for callers with their own edge kernels (sngDbscan).
@@ -263,13 +282,25 @@ int launch_uf_compress(const ClusterArgs& a, cudaStream_t st) {
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
+int launch_uf_compress_round(int n, const uint8_t* core, int32_t* parent, cudaStream_t st) {
+    if (n < kCompressRounds) return 0;
+    ClusterArgs a{};
+    a.n = n;
+    a.core = core;
+    a.parent = parent;
+    return launch_uf_compress(a, st);
+}
+
 int launch_cluster_labels(const ClusterArgs& a, cudaStream_t st) {
-    k_root_flags<<<(a.n + 1 + 255) / 256, 256, 0, st>>>(a);
-    if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    const int r = launch_scan_i64(a.rootFlag, a.rootFlag, (size_t)a.n + 1, a.scanTmp, st);
+    const RootFlags flags{a.core, a.parent, a.n};
+    const size_t n1 = (size_t)a.n + 1, nb = scan::tiles(n1);
+    // the tiles' offsets are added by the labels where a block can hold them
+    const bool local = n1 > scan::kScanOne && nb <= scan::kSumsInSmem;
+    const int r = local ? scan::launch_local(flags, a.rootFlag, n1, a.scanTmp, st)
+                        : scan::launch(flags, a.rootFlag, n1, a.scanTmp, st);
     if (r < 0) return -1;
-    k_labels<<<(a.n + 255) / 256, 256, 0, st>>>(a);
-    return cudaPeekAtLastError() == cudaSuccess ? r + 2 : -1;
+    k_labels<<<(a.n + scan::kThreads - 1) / scan::kThreads, scan::kThreads, 0, st>>>(a, a.scanTmp, local ? (int)nb : 0);
+    return cudaPeekAtLastError() == cudaSuccess ? r + 1 : -1;
 }
 
 }  // namespace sdb

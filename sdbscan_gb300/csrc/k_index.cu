@@ -11,7 +11,7 @@
 // Hub lists: for every point, the top-m lists that contain it.  A point in no
 // list ("non-hub") can never be a candidate of anyone, so its neighbourhood
 // is exactly its own candidates within eps.
-#include "common.cuh"
+#include "scan.cuh"
 
 #include <algorithm>
 
@@ -80,15 +80,18 @@ __global__ void k_index_scatter(IndexArgs a) {
     }
 }
 
-// Tile order: counting sort of the tiles by the chunk of their first member.
-__global__ void k_tile_keys(IndexArgs a) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.tileOff[2 * a.nproj]) return;
-    const int l = a.tileList[t];
-    const int mt = (int)((t - a.tileOff[l]) / a.nct);
-    const int key = a.members[a.listOff[l] + (int64_t)mt * a.TM].x / a.chunkPts;
-    a.tileKey[t] = key;
-    atomicAdd(reinterpret_cast<unsigned long long*>(a.keyOff) + key, 1ull);
+// A block per list: its tiles' list ids, and the keys of the tile order, a
+// counting sort of the tiles by the chunk of their first member.
+__global__ void __launch_bounds__(64) k_tile_keys(IndexArgs a) {
+    const int l = blockIdx.x;
+    const int64_t t0 = a.tileOff[l], t1 = a.tileOff[l + 1];
+    for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+        a.tileList[t] = l;
+        const int64_t mt = (t - t0) / a.nct;
+        const int key = a.members[a.listOff[l] + mt * a.TM].x / a.chunkPts;
+        a.tileKey[t] = key;
+        atomicAdd(reinterpret_cast<unsigned long long*>(a.keyOff) + key, 1ull);
+    }
 }
 
 // The tensor-core distance kernel's order: tiles by (super-chunk of their
@@ -122,19 +125,14 @@ __global__ void k_tile_perm(IndexArgs a) {
     a.tilePerm[pos] = (int32_t)t;
 }
 
-// tiles per list -> listCount reused as the tile count input of the scan
-__global__ void k_tile_counts(IndexArgs a, int64_t* tiles) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= 2 * a.nproj) return;
-    const int64_t members = a.listOff[l + 1] - a.listOff[l];
-    tiles[l] = ((members + a.TM - 1) / a.TM) * a.nct;
-}
-
-__global__ void k_tile_fill(IndexArgs a) {
-    const int l = blockIdx.x;
-    const int64_t t0 = a.tileOff[l], t1 = a.tileOff[l + 1];
-    for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) a.tileList[t] = l;
-}
+// Tiles of a list, the input of the tile offsets' scan.
+struct TileCounts {
+    const int64_t* listOff;
+    int L, TM, nct;
+    __device__ int64_t operator()(size_t l) const {
+        return l < (size_t)L ? (listOff[l + 1] - listOff[l] + TM - 1) / TM * nct : 0;
+    }
+};
 
 __global__ void k_hubs_count(IndexArgs a) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -158,94 +156,23 @@ __global__ void k_pad_copy(const float* __restrict__ X, int n, int d, float* __r
     Xt[q] = c < d ? X[(size_t)p * d + c] : 0.0f;
 }
 
-__global__ void k_i32_to_i64(const int32_t* in, int64_t* out, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[i];
-}
-
-// ---- exclusive scan of int64 (three phases, recursive on block sums) -------
-constexpr int kScanBlock = 256, kScanItems = 4, kScanTile = kScanBlock * kScanItems;
-
-__device__ int64_t block_exclusive(int64_t v, int64_t* total) {
-    __shared__ int64_t wsum[kScanBlock / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int64_t x = v;
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-        const int64_t o = __shfl_up_sync(0xffffffffu, x, s);
-        if (lane >= s) x += o;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int64_t y = lane < kScanBlock / 32 ? wsum[lane] : 0;
-#pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
-            const int64_t o = __shfl_up_sync(0xffffffffu, y, s);
-            if (lane >= s) y += o;
-        }
-        if (lane < kScanBlock / 32) wsum[lane] = y;
-    }
-    __syncthreads();
-    const int64_t before = w ? wsum[w - 1] : 0;
-    *total = wsum[kScanBlock / 32 - 1];
-    __syncthreads();
-    return before + x - v;
-}
-
-__global__ void k_scan_tiles(const int64_t* in, int64_t* out, size_t n, int64_t* sums) {
-    const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-    int64_t v[kScanItems], s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        v[i] = base + i < n ? in[base + i] : 0;
-        s += v[i];
-    }
-    int64_t total;
-    int64_t ex = block_exclusive(s, &total);
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        if (base + i < n) out[base + i] = ex;
-        ex += v[i];
-    }
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void k_scan_add(int64_t* out, size_t n, const int64_t* offs) {
-    const size_t i = (size_t)blockIdx.x * kScanTile + threadIdx.x;
-    const int64_t o = offs[blockIdx.x];
-    for (int t = 0; t < kScanItems; ++t) {
-        const size_t j = i + (size_t)t * kScanBlock;
-        if (j < n && j < (size_t)(blockIdx.x + 1) * kScanTile) out[j] += o;
-    }
-}
-
 }  // namespace
 
 size_t scan_tmp_elems(size_t n) {
     size_t tot = 0;
     while (n > 1) {
-        const size_t nb = (n + kScanTile - 1) / kScanTile;
-        tot += nb + 1;
-        n = nb;
+        n = scan::tiles(n);
+        tot += n + 1;
     }
     return tot + 2;
 }
 
 int launch_scan_i64(const int64_t* in, int64_t* out, size_t n, int64_t* tmp, cudaStream_t st) {
-    if (n == 0) return 0;
-    const size_t nb = (n + kScanTile - 1) / kScanTile;
-    int launches = 0;
-    k_scan_tiles<<<(unsigned)nb, kScanBlock, 0, st>>>(in, out, n, tmp);
-    ++launches;
-    if (nb > 1) {
-        int r = launch_scan_i64(tmp, tmp, nb, tmp + nb + 1, st);
-        if (r < 0) return -1;
-        launches += r;
-        k_scan_add<<<(unsigned)nb, kScanBlock, 0, st>>>(out, n, tmp);
-        ++launches;
-    }
-    return cudaPeekAtLastError() == cudaSuccess ? launches : -1;
+    return scan::launch(scan::Load64{in}, out, n, tmp, st);
+}
+
+int launch_scan_i32(const int32_t* in, size_t n, int64_t* out, int64_t* tmp, cudaStream_t st) {
+    return scan::launch(scan::Load32{in, n}, out, n + 1, tmp, st);
 }
 
 int launch_index_count(const IndexArgs& a, cudaStream_t st) {
@@ -267,7 +194,7 @@ int launch_tile_order(const IndexArgs& a, cudaStream_t st) {
     if (a.maxTiles <= 0) return 0;
     if (cudaMemsetAsync(a.keyOff, 0, sizeof(int64_t) * ((size_t)a.nChunks + 1), st) != cudaSuccess) return -1;
     const unsigned g = (unsigned)((a.maxTiles + 255) / 256);
-    k_tile_keys<<<g, 256, 0, st>>>(a);
+    k_tile_keys<<<2 * a.nproj, 64, 0, st>>>(a);
     if (cudaPeekAtLastError() != cudaSuccess) return -1;
     const int r = launch_scan_i64(a.keyOff, a.keyOff, (size_t)a.nChunks + 1, a.scanTmp, st);
     if (r < 0) return -1;
@@ -293,19 +220,10 @@ int launch_tile_order_list(const IndexArgs& a, int superChunk, int32_t* keys, in
     return cudaPeekAtLastError() == cudaSuccess ? r + 2 : -1;
 }
 
-// Computes tileOff (scan of per-list tile counts) into a.tileOff; tile counts
-// are staged in a.listCount (free by then).
+// tileOff: the lists' tile counts, scanned.
 int launch_tile_offsets(const IndexArgs& a, cudaStream_t st) {
     const int L = 2 * a.nproj;
-    k_tile_counts<<<(L + 255) / 256, 256, 0, st>>>(a, a.listCount);
-    if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    int r = launch_scan_i64(a.listCount, a.tileOff, (size_t)L + 1, a.scanTmp, st);
-    return r < 0 ? -1 : r + 1;
-}
-
-int launch_tiles(const IndexArgs& a, int64_t, cudaStream_t st) {
-    k_tile_fill<<<2 * a.nproj, 256, 0, st>>>(a);
-    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+    return scan::launch(TileCounts{a.listOff, L, a.TM, a.nct}, a.tileOff, (size_t)L + 1, a.scanTmp, st);
 }
 
 int launch_hubs_count(const IndexArgs& a, cudaStream_t st) {
@@ -323,11 +241,6 @@ int launch_hubs_scatter(const IndexArgs& a, cudaStream_t st) {
 int launch_pad_copy(const float* X, int n, int d, float* Xt, int ld, cudaStream_t st) {
     const size_t total = (size_t)n * ld;
     k_pad_copy<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(X, n, d, Xt, ld);
-    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
-}
-
-int launch_i32_to_i64(const int32_t* in, int64_t* out, int n, cudaStream_t st) {
-    k_i32_to_i64<<<(n + 255) / 256, 256, 0, st>>>(in, out, n);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 

@@ -24,17 +24,12 @@ __global__ void k_csr_hook(CsrArgs a, int from) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p]) return;
     const int64_t e0 = a.off[p], len = a.off[p + 1] - e0;
-    RootSpan span(load_parent(a.parent, p));
+    RootSpan span(round_root(a.parent, p, a.n));
     for (int t = from; t < from + 4 && t < len; ++t) {
         const int q = __ldg(a.idx + e0 + t);
-        if (a.core[q]) span.see(load_parent(a.parent, q));
+        if (a.core[q]) span.see(round_root(a.parent, q, a.n));
     }
     span.hook(a.parent);
-}
-
-__global__ void k_csr_compress(CsrArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < a.n && a.core[p]) a.parent[p] = find_root(a.parent, p);
 }
 
 // A warp per core point over its smaller core neighbours (each edge once).
@@ -94,12 +89,18 @@ __global__ void __launch_bounds__(256) k_csr_edges(CsrArgs a) {
 int launch_csr_starts(const CsrArgs& a, cudaStream_t st) {
     const int g = (a.n + 255) / 256;
     int launches = 0;
-    for (int t = 0; t < 3; ++t, launches += 2) {
+    for (int t = 0; t < 3; ++t, ++launches) {
         k_csr_hook<<<g, 256, 0, st>>>(a, 4 * t);
-        k_csr_compress<<<g, 256, 0, st>>>(a);
+        const int r = launch_uf_compress_round(a.n, a.core, a.parent, st);
+        if (r < 0) return -1;
+        launches += r;
     }
     k_csr_union<<<(a.n + 7) / 8, 256, 0, st>>>(a);
-    k_csr_compress<<<g, 256, 0, st>>>(a);
+    ClusterArgs ka{};
+    ka.n = a.n;
+    ka.core = a.core;
+    ka.parent = a.parent;
+    if (launch_uf_compress(ka, st) < 0) return -1;
     k_csr_start<<<g, 256, 0, st>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? launches + 3 : -1;
 }

@@ -208,12 +208,12 @@ __global__ void __launch_bounds__(256) k_sng_hook(SngArgs a, const uint8_t* __re
                                                   int word0) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !core[p]) return;
-    RootSpan span(load_parent(parent, p));
+    RootSpan span(round_root(parent, p, a.n));
     for (int ct = word0; ct < min(word0 + 2, a.nct); ++ct) {
         uint64_t w = __ldg(reinterpret_cast<const unsigned long long*>(a.mask) + (size_t)ct * a.n + p);
         for (int c = 0; c < 2 && w; ++c, w &= w - 1) {
             const int q = __ldg(a.cols + ct * kTNK + __ffsll((long long)w) - 1);
-            if (core[q]) span.see(load_parent(parent, q));
+            if (core[q]) span.see(round_root(parent, q, a.n));
         }
     }
     span.hook(parent);
@@ -392,14 +392,11 @@ int launch_sng_degree(const SngArgs& a, int exact, int optics, int minPts, int32
 int launch_sng_union(const SngArgs& a, const uint8_t* core, int32_t* parent, cudaStream_t st) {
     int launches = 0;
     if (a.nct > 0) {
-        ClusterArgs ka{};
-        ka.n = a.n;
-        ka.core = core;
-        ka.parent = parent;
-        for (int t = 0; t < 3; ++t) {
+        for (int t = 0; t < 3; ++t, ++launches) {
             k_sng_hook<<<(a.n + 255) / 256, 256, 0, st>>>(a, core, parent, 2 * t);
-            if (launch_uf_compress(ka, st) < 0) return -1;
-            launches += 2;
+            const int r = launch_uf_compress_round(a.n, core, parent, st);
+            if (r < 0) return -1;
+            launches += r;
         }
         k_sng_union<<<dim3((a.n + 255) / 256, (a.nct + kGroup - 1) / kGroup), 256, 0, st>>>(a, core, parent);
         ++launches;

@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(256) k_sngb_hook(SngBlockArgs a, const uint8_t
     const int lane = (int)lane_id();
     const int64_t p = b * BR + lane;
     if (p >= a.n || !core[p]) return;
-    RootSpan span(load_parent(parent, (int)p));
+    RootSpan span(round_root(parent, (int)p, a.n));
     int seen = 0;
     for (int64_t j = j0; j < min(j0 + 64, a.S) && seen < 3; ++j) {
         if (!((__ldg(a.words + b * a.S + j) >> lane) & 1u)) continue;
         const int q = block_draw(a.key, a.S, b, j, a.n);
         if (!core[q]) continue;
-        span.see(load_parent(parent, q));
+        span.see(round_root(parent, q, a.n));
         ++seen;
     }
     span.hook(parent);
@@ -319,16 +319,15 @@ int launch_sngb_pass(const SngBlockArgs& a, int minPts, uint8_t* core, cudaStrea
 }
 
 int launch_sngb_union(const SngBlockArgs& a, const uint8_t* core, int32_t* parent, cudaStream_t st) {
-    ClusterArgs ka{};
-    ka.n = a.n;
-    ka.core = core;
-    ka.parent = parent;
+    int launches = 4;
     for (int t = 0; t < 3; ++t) {
         k_sngb_hook<<<(a.n + 255) / 256, 256, 0, st>>>(a, core, parent, 64 * t);
-        if (launch_uf_compress(ka, st) < 0) return -1;
+        const int r = launch_uf_compress_round(a.n, core, parent, st);
+        if (r < 0) return -1;
+        launches += r;
     }
     k_sngb_union<<<grid_spans(a), 256, 0, st>>>(a, core, parent);
-    return cudaPeekAtLastError() == cudaSuccess ? 7 : -1;
+    return cudaPeekAtLastError() == cudaSuccess ? launches : -1;
 }
 
 int launch_sngb_border(const SngBlockArgs& a, const uint8_t* core, const int32_t* parent, int32_t* border,

@@ -13,7 +13,7 @@
 //     in it.
 //  3. An exact sort of each candidate list by (value desc, point asc) yields
 //     the top m (k_select).  A list whose candidates overflow its buffer is
-//     resolved by an exact radix select over the whole column (k_fallback).
+//     resolved by an exact radix select over the whole column (select_column).
 // Ties: the reference's heap keeps, among equal values at the boundary, the
 // ones its heap order dictates; this engine keeps the smallest point ids and
 // counts such boundary ties.
@@ -174,36 +174,15 @@ __global__ void k_collect1(TopMArgs a) {
     }
 }
 
-// One CTA per list: exact sort of the candidates, first m written to topM.
-__global__ void k_select(TopMArgs a) {
-    extern __shared__ uint64_t sk[];
-    const int list = blockIdx.x;
-    const int r = list % a.nproj, side = list / a.nproj;
-    const int c = a.candCount[list];
-    if (c > a.cap) return;  // resolved by k_fallback
-    const int len = pow2_ceil(max(c, 2));
-    for (int i = threadIdx.x; i < len; i += blockDim.x) sk[i] = i < c ? a.cand[(size_t)list * a.cap + i] : 0ull;
-    block_sort_desc(sk, len);
-    // c >= m always holds (the threshold is attained by >= m points); if it
-    // ever did not, point 0 stands in and the fit reports an internal error.
-    for (int i = threadIdx.x; i < a.m; i += blockDim.x)
-        a.topM[(size_t)r * 2 * a.m + side * a.m + i] = i < c ? (int32_t)(0xffffffffu - (uint32_t)sk[i]) : 0;
-    if (threadIdx.x == 0 && c < a.m) atomicExch(a.errFlag, 1);
-    if (threadIdx.x == 0 && c > a.m && (sk[a.m - 1] >> 32) == (sk[a.m] >> 32)) atomicAdd(a.ties, 1ull);
-}
-
 // Exact radix select over a whole column, for lists whose candidate buffer
-// overflowed (heavy ties, adversarial orderings).  One CTA per list; CTAs of
-// lists that did not overflow return at once.
-__global__ void k_fallback(TopMArgs a) {
+// overflowed (heavy ties, adversarial orderings).  sk: shared memory, m entries
+// rounded up to a power of two.
+__device__ void select_column(const TopMArgs& a, int list, uint64_t* sk) {
     __shared__ uint32_t hist[256];
     __shared__ uint32_t prefix, prefixMask;
     __shared__ int need;  // how many of the remaining (prefix-matching) elements we still take
     __shared__ int above; // elements strictly above the final key
     __shared__ int taken;
-    extern __shared__ uint64_t sk[];  // m (pow2) selected entries
-    const int list = blockIdx.x;
-    if (a.candCount[list] <= a.cap) return;
     const int r = list % a.nproj, side = list / a.nproj;
     auto keyAt = [&](int p) -> uint32_t {
         const float v = a.P[(size_t)p * a.nproj + r];
@@ -285,6 +264,27 @@ __global__ void k_fallback(TopMArgs a) {
     if (threadIdx.x == 0 && eqTotal > need) atomicAdd(a.ties, 1ull);
 }
 
+// One CTA per list: exact sort of the candidates, first m written to topM.
+__global__ void k_select(TopMArgs a) {
+    extern __shared__ uint64_t sk[];
+    const int list = blockIdx.x;
+    const int r = list % a.nproj, side = list / a.nproj;
+    const int c = a.candCount[list];
+    if (c > a.cap) {
+        select_column(a, list, sk);
+        return;
+    }
+    const int len = pow2_ceil(max(c, 2));
+    for (int i = threadIdx.x; i < len; i += blockDim.x) sk[i] = i < c ? a.cand[(size_t)list * a.cap + i] : 0ull;
+    block_sort_desc(sk, len);
+    // c >= m always holds (the threshold is attained by >= m points); if it
+    // ever did not, point 0 stands in and the fit reports an internal error.
+    for (int i = threadIdx.x; i < a.m; i += blockDim.x)
+        a.topM[(size_t)r * 2 * a.m + side * a.m + i] = i < c ? (int32_t)(0xffffffffu - (uint32_t)sk[i]) : 0;
+    if (threadIdx.x == 0 && c < a.m) atomicExch(a.errFlag, 1);
+    if (threadIdx.x == 0 && c > a.m && (sk[a.m - 1] >> 32) == (sk[a.m] >> 32)) atomicAdd(a.ties, 1ull);
+}
+
 }  // namespace
 
 int launch_topm_thresholds(const TopMArgs& a, cudaStream_t st) {
@@ -319,10 +319,7 @@ int launch_topm_select(const TopMArgs& a, cudaStream_t st) {
         cudaFuncSetAttribute(k_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
         return -1;
     k_select<<<2 * a.nproj, 256, sm, st>>>(a);
-    if (cudaPeekAtLastError() != cudaSuccess) return -1;
-    const size_t sm2 = sizeof(uint64_t) * pow2_ceil(a.m < 2 ? 2 : a.m);
-    k_fallback<<<2 * a.nproj, 256, sm2, st>>>(a);
-    return cudaPeekAtLastError() == cudaSuccess ? 2 : -1;
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
 }  // namespace sdb

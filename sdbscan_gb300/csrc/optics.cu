@@ -27,7 +27,6 @@ namespace sdb {
 int launch_core_emit(const CoreArgs& a, const void* sig, const int64_t* nbOff, int32_t* nbIdx, float* nbDist,
                      int32_t* nbFill, cudaStream_t st);
 int launch_core_dist(const CoreArgs& a, const int64_t* nbOff, const float* nbDist, cudaStream_t st);
-int launch_i32_to_i64(const int32_t* in, int64_t* out, int n, cudaStream_t st);
 }  // namespace sdb
 
 using namespace sdb;
@@ -129,16 +128,11 @@ struct Floods {
 sdb_status sdb_engine::optics_stage(const CoreArgs& ca, int& launches) {
     cudaStream_t st = stream;
     if (!ensure(nbOff, sizeof(int64_t) * (n + 1)) || !ensure(nbFill, sizeof(int32_t) * n)) return SDB_ERR_NOMEM;
-    cudaError_t e = cudaMemsetAsync(nbOff.ptr, 0, sizeof(int64_t) * (n + 1), st);
-    if (e != cudaSuccess) return cuda_fail(e, "memset");
-    int r = launch_i32_to_i64(ca.degree, i64(nbOff), n, st);
-    if (r < 0) return fail(SDB_ERR_CUDA, "degree conversion launch failed");
-    launches += r;
-    r = launch_scan_i64(i64(nbOff), i64(nbOff), (size_t)n + 1, i64(scanTmp), st);
+    int r = launch_scan_i32(ca.degree, n, i64(nbOff), i64(scanTmp), st);
     if (r < 0) return fail(SDB_ERR_CUDA, "scan launch failed");
     launches += r;
     int64_t total = 0;
-    e = cudaMemcpyAsync(&total, i64(nbOff) + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(&total, i64(nbOff) + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "neighbour count");
     if (!ensure(nbIdx, sizeof(int32_t) * std::max<int64_t>(total, 1)) ||

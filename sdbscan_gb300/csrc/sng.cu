@@ -43,13 +43,14 @@
 #include "engine_internal.h"
 
 namespace sdb {
-int launch_i32_to_i64(const int32_t* in, int64_t* out, int n, cudaStream_t st);
 int launch_core_dist(const CoreArgs& a, const int64_t* nbOff, const float* nbDist, cudaStream_t st);
 }  // namespace sdb
 
 using namespace sdb;
 
 namespace {
+
+constexpr int64_t kMinPackedDraws = 384;
 
 struct SngSample {
     std::vector<int32_t> cols, mult;  // distinct drawn ids (ascending) and their draw counts
@@ -313,9 +314,7 @@ sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float*
     }
     if (optics) {
         // distinct neighbour lists: offsets from the degrees, then the pairs again
-        SDB_CK(cudaMemsetAsync(nbOff.ptr, 0, sizeof(int64_t) * (n + 1), st));
-        L_(launch_i32_to_i64(i32(degree), i64(nbOff), n, st));
-        L_(launch_scan_i64(i64(nbOff), i64(nbOff), (size_t)n + 1, i64(scanTmp), st));
+        L_(launch_scan_i32(i32(degree), n, i64(nbOff), i64(scanTmp), st));
         if (!ok) return fail(SDB_ERR_CUDA, "neighbour offsets launch failed");
         int64_t total = 0;
         SDB_CK(cudaMemcpyAsync(&total, i64(nbOff) + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -398,7 +397,11 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
           ensure(labels, sizeof(int32_t) * n) && ensure(nClusters, sizeof(int32_t) * 4) &&
           ensure(scanTmp, sizeof(int64_t) * scan_tmp_elems((size_t)n + 1)) &&
           ensure(sngWords, sizeof(uint32_t) * std::max<size_t>(1, (size_t)nb * (size_t)std::max<int64_t>(S, 0)));
-    const size_t copyBytes = S > 0 ? sng_pair_bytes(p.distance, n, ld) : 0;
+    // the packed tile reads a copy of all points: worth it from kMinPackedDraws
+    // draws per point on (50K x 64, 250 draws: 0.35 ms with, 0.33 without; 50K x
+    // 784, 500 draws, pass and copy: 0.87 and 0.99), and for sngOptics always,
+    // which keeps its distances
+    const size_t copyBytes = S > 0 && (optics || S >= kMinPackedDraws) ? sng_pair_bytes(p.distance, n, ld) : 0;
     const bool packed = copyBytes > 0 && !noCandCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
                         (p.distance != SDB_CHI2 || ensure(smallEntry, n));
     // sngOptics keeps the pass's distances for its emitting pass
@@ -489,9 +492,7 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
         L_(launch_sngb_emit(ba, st));
         SDB_CK(cudaEventRecord(ev[5], st));
         L_(launch_sngb_distinct(ba, minPts, i32(degree), static_cast<uint8_t*>(core.ptr), st));
-        SDB_CK(cudaMemsetAsync(nbOff.ptr, 0, sizeof(int64_t) * (n + 1), st));
-        L_(launch_i32_to_i64(i32(degree), i64(nbOff), n, st));
-        L_(launch_scan_i64(i64(nbOff), i64(nbOff), (size_t)n + 1, i64(scanTmp), st));
+        L_(launch_scan_i32(i32(degree), n, i64(nbOff), i64(scanTmp), st));
         if (!ok) return fail(SDB_ERR_CUDA, "sampled-block launch failed");
         int64_t total = 0;
         SDB_CK(cudaMemcpyAsync(&total, i64(nbOff) + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));

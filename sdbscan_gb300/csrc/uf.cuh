@@ -35,6 +35,13 @@ static __device__ void unite(int32_t* parent, int a, int b) {
     }
 }
 
+// The root a hooking round starts from: found by walking, or, where the paths
+// were compressed before the round (n >= kCompressRounds), the parent as it is
+// (an ancestor if not the root).
+static __device__ __forceinline__ int round_root(int32_t* parent, int x, int n) {
+    return n >= kCompressRounds ? load_parent(parent, x) : find_root(parent, x);
+}
+
 // Hooking without unites: a point that saw the roots r (its own) and others of
 // its component hooks the largest of them and its own under the smallest, by
 // plain atomicMin.  Parents only move down, so the forest stays a forest; where
