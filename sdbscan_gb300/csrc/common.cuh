@@ -96,7 +96,8 @@ struct ProjectArgs {
     int fhtDim, nproj, k;
     float* P;            // n x nproj projections out
     int32_t* topK;       // n x 2k out
-    uint32_t* chunkExt;  // G x nproj: (max v, max -v) of the chunk, BF16 rounded down, v in the low half
+    uint32_t* chunkExt;  // G x nproj: (max v, max -v) of the chunk as BF16 bits, v in the low half; the top 16
+                         // bits of the order-preserving key are at most the extreme's
     int chunk;           // points per chunk (G = ceil(n / chunk))
     int chunkBase, chunkEnd;  // chunks this launch covers (chunkEnd 0: all G)
     int32_t* err;        // device flags: [0] negative input, [1] zero point

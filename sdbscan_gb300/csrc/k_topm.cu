@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThrThreads) k_thresholds(TopMArgs a, int cols
                 }
                 if (warp_sum(cnt) >= a.m) t = at;
             }
-            t = (t << 16) | (t & 0x8000u ? 0u : 0xffffu);  // the value's 32-bit key
+            t <<= 16;  // the smallest 32-bit key with these high bits
         }
         if (lane == 0) (side ? a.thrMin : a.thrMax)[rr] = __uint_as_float(t);  // raw key bits
     }
