@@ -54,8 +54,8 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
 // restores a link that two hooks of one root lost.  With every point a set of
 // its own the tile pass would send some twenty unites per point at the same few
 // roots, all at once; after the rounds it finds almost nothing but equal roots
-// (50K x 128: union 379 us without, 35 plus 45 for the rounds; 1M x 784: 1827
-// and 613 + 263; hooking only the own root left 100 and 955).
+// (1M x 784: union 1827 us without, 291 + 263 for the rounds; hooking only the
+// own root left 955, walking to the members' roots first 613).
 __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p] || (a.carry && a.coreEps[p] != a.round)) return;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_union_tiles(ClusterArgs a) {
     }
     __syncthreads();
     if (!bits) return;
-    int rp = find_root(a.parent, p);
+    int rp = load_parent(a.parent, p);  // the root mostly; an ancestor proves the same set as well
     const int ng = groups;
     for (int g = 0; g < ng; ++g) {
         const int cr = reinterpret_cast<volatile int&>(group[g].root);
