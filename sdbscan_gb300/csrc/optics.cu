@@ -162,8 +162,18 @@ sdb_status sdb_engine::optics_order(int64_t total) {
     cudaError_t e = cudaSuccess;
     if (!ensure(parent, sizeof(int32_t) * n) || !ensure(border, sizeof(int32_t) * n) ||
         !ensure(floodStart, sizeof(int32_t) * n) || !ensure(newId, sizeof(int32_t) * n) ||
-        !ensure(edgeOff, sizeof(int64_t) * (n + 1)) || !ensure(edges, sizeof(Edge) * std::max<int64_t>(total, 1)))
+        !ensure(edgeOff, sizeof(int64_t) * (n + 1)))
         return SDB_ERR_NOMEM;
+    const size_t edgeBytes = sizeof(Edge) * std::max<int64_t>(total, 1);
+    if (!ensure(edges, edgeBytes)) {
+        // the lists are made: what only the distance stage reads makes room
+        // (the distances alone are n x 2k x m floats)
+        e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return cuda_fail(e, "neighbour lists");
+        release(dists);
+        release(candT);
+        if (!ensure(edges, edgeBytes)) return SDB_ERR_NOMEM;
+    }
     CsrArgs a{};
     a.n = n;
     a.core = static_cast<const uint8_t*>(core.ptr);

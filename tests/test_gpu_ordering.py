@@ -52,3 +52,43 @@ def test_ordering_matches_oracle(n, d, c, spread, eps, minPts, order):
     np.testing.assert_array_equal(e.optics()[0], o_order)
     np.testing.assert_array_equal(e.optics()[1], o_reach)
     e.close()
+
+
+def test_ordering_takes_the_distances_memory_when_there_is_no_other():
+    """The floods' copy of the lists fits where the pair distances were: the
+    fit needs the two list arrays (8 bytes an entry) beyond a fit without
+    entries, and less than that plus the copy (16 bytes an entry)."""
+    from sdbscan_gb300 import capi
+    n, d = 600, 12
+    X = _clusters(n, d, 12, 0.25, 5, "mixed")
+
+    def fit(eps, cap=0):
+        e = capi.Engine(n, d)
+        e.set_params(n_proj=256, topK=3, topM=50, random_seed=4)
+        e.set_debug_limits(device_bytes_cap=cap)
+        try:
+            e.fit_soptics(X, eps, 2)
+            return e.optics() + (int(e.core()[1].sum()),)
+        finally:
+            e.close()
+
+    def smallest_cap(eps):
+        lo, hi = 1 << 16, 1 << 28
+        while hi - lo > 1 << 12:
+            mid = (lo + hi) // 2
+            try:
+                fit(eps, mid)
+                hi = mid
+            except capi.SdbError as err:
+                assert err.status == 6
+                lo = mid
+        return hi
+
+    eps = 0.05
+    order, reach, entries = fit(eps)
+    assert 5000 < entries and 8 * entries < 4 * n * 6 * 50  # the copy is smaller than the distances
+    cap = smallest_cap(eps)
+    assert cap - smallest_cap(1e-9) < 12 * entries
+    got = fit(eps, cap)
+    np.testing.assert_array_equal(got[0], order)
+    np.testing.assert_array_equal(got[1], reach)
