@@ -119,7 +119,10 @@ int launch_transform(const ProjectArgs& a, cudaStream_t st);
 
 // Random Fourier features for L1/L2: E[p] = [cos(R x_p), sin(R x_p)].
 // gate (optional): run only if *gate != 0 (the tensor-core embedding failed).
-int launch_rff(const float* Xt, int ld, int n, int d, const float* R, int h, float* E, cudaStream_t st,
+// floats of the dimension-major copy of R, the copy, and the embedding from it
+size_t rff_tile_floats(int h, int ld);
+int launch_rff_tiles(const float* Rt, int ld, int h, float* tiles, cudaStream_t st);
+int launch_rff(const float* Xt, int ld, int n, const float* Rtiles, int h, float* E, cudaStream_t st,
                const int32_t* gate = nullptr);
 // BF16 mode: the same embedding on the tensor cores from split-BF16 copies
 // ([hi | lo] per row) of the points (n x 2 ldb) and of R (h x 2 ldb); err set

@@ -129,7 +129,7 @@ std::vector<DevBuf*> sdb_engine::all_bufs() {
             &sngExtraPass, &sngMask, &rowDeg, &colCnt, &sngUb, &sngHeavy, &chunkOff, &tileKey, &keyOff, &tilePerm,
             &Cb, &candT, &tileKeyTc, &keyOffTc, &tilePermTc, &sngWords, &hashOffB, &hashIdB, &hashDistB, &sqNorm, &multiMask,
             &multiIdx, &slotMulti, &slotHub, &hubPoint, &smallEntry,
-            &floodStart, &newId, &edgeOff, &edges};
+            &floodStart, &newId, &edgeOff, &edges, &RtTiles};
 }
 
 // ---------------------------------------------------------------------------
@@ -312,7 +312,8 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
           ensure(slotMulti, sizeof(int32_t) * (size_t)L * m) && ensure(slotHub, sizeof(int32_t) * (size_t)L * m);
     if (optics) ok &= ensure(sig, 16 * (size_t)L * m);
     if (pairTiles && p.distance == SDB_CHI2) ok &= ensure(smallEntry, n);
-    if (rff) ok &= ensure(E, sizeof(float) * (size_t)n * ker) && ensure(Rt, sizeof(float) * hostRt.size());
+    if (rff) ok &= ensure(E, sizeof(float) * (size_t)n * ker) && ensure(Rt, sizeof(float) * hostRt.size()) &&
+                   ensure(RtTiles, sizeof(float) * rff_tile_floats(ker / 2, ld));
     if (optics || sweep) ok &= ensure(dists, sizeof(float) * (size_t)n * 2 * k * m);
     if (optics) ok &= ensure(coreDist, sizeof(float) * n);
     if (!ok) return SDB_ERR_NOMEM;
@@ -388,6 +389,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
             SDB_CK(cudaMemcpyAsync(Rt.ptr, hostRt.data(), sizeof(float) * hostRt.size(), cudaMemcpyHostToDevice, st));
         L_(launch_pad_copy(Xd, n, d, f32(Xt), ld, st));
         const int h = ker / 2;
+        L_(launch_rff_tiles(f32(Rt), ld, h, f32(RtTiles), st));
         int tcr = -1;
         if (p.precision == SDB_PREC_BF16) {
             // the embedding GEMM on the tensor cores from split-BF16 copies of X
@@ -400,7 +402,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
             tcr = launch_rff_tc(Xb.ptr, Rb.ptr, n, h, ldb, f32(E), i32(errFlags) + 5, dbgStallSpins, st);
             if (tcr > 0) launches += tcr;
         }
-        L_(launch_rff(f32(Xt), ld, n, d, f32(Rt), h, f32(E), st, tcr > 0 ? i32(errFlags) + 5 : nullptr));
+        L_(launch_rff(f32(Xt), ld, n, f32(RtTiles), h, f32(E), st, tcr > 0 ? i32(errFlags) + 5 : nullptr));
         pa.X = f32(Xt);
         pa.ldx = ld;
         pa.E = f32(E);

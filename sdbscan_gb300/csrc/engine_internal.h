@@ -88,7 +88,7 @@ struct sdb_engine {
         coreEps, sampleFlag, noiseFlag, noiseCores, noisePts, PcT, numCore, pairRound, sngCols, sngMult, sngColOf,
         sngExtras, sngExtraPass, sngMask, rowDeg, colCnt, sngUb, sngHeavy, chunkOff, tileKey, keyOff, tilePerm, Cb, candT,
         tileKeyTc, keyOffTc, tilePermTc, sngWords, hashOffB, hashIdB, hashDistB, sqNorm, multiMask, multiIdx, slotMulti,
-        slotHub, hubPoint, smallEntry, floodStart, newId, edgeOff, edges;
+        slotHub, hubPoint, smallEntry, floodStart, newId, edgeOff, edges, RtTiles;
 
     // results
     bool haveLabels = false, haveOptics = false, haveFit = false, lastOptics = false;
