@@ -54,86 +54,89 @@ __global__ void __launch_bounds__(16 * TX, (dist_min_blocks<TX, CN, KT, NST>()))
     __shared__ int passTotal;
 
     const int tid = threadIdx.x;
-    if ((int64_t)blockIdx.x >= *a.tileTotal) return;
-    const int64_t t = tile_at(a.tilePerm, blockIdx.x);
-    const int l = a.tileList[t];
-    const int64_t ti = t - a.tileOff[l];
-    const int mt = (int)(ti / a.nct), ct = (int)(ti % a.nct);
-    const int64_t mbeg = a.listOff[l] + (int64_t)mt * TM;
-    const int64_t mend = a.listOff[l + 1];
-    const int r = l % a.nproj, side = l / a.nproj;
-    const int32_t* cand = a.topM + (size_t)r * 2 * a.m + side * a.m;
+    const int64_t tiles = *a.tileTotal;
+    for (int64_t b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int64_t t = tile_at(a.tilePerm, b);
+        const int l = a.tileList[t];
+        const int64_t ti = t - a.tileOff[l];
+        const int mt = (int)(ti / a.nct), ct = (int)(ti % a.nct);
+        const int64_t mbeg = a.listOff[l] + (int64_t)mt * TM;
+        const int64_t mend = a.listOff[l + 1];
+        const int r = l % a.nproj, side = l / a.nproj;
+        const int32_t* cand = a.topM + (size_t)r * 2 * a.m + side * a.m;
 
-    for (int i = tid; i < TM; i += NT) {
-        const int64_t q = mbeg + i;
-        if (q < mend) {
-            const int2 mb = a.members[q];
-            rowPoint[i] = mb.x;
-            rowSlot[i] = mb.y;
-        } else {
-            rowPoint[i] = -1;
-            rowSlot[i] = 0;
-        }
-        smask[2 * i] = 0;
-        smask[2 * i + 1] = 0;
-    }
-    for (int j = tid; j < TNK; j += NT) {
-        const int c = ct * TN + j;
-        colPoint[j] = c < a.m ? cand[c] : -1;
-        colCount[j] = 0;
-    }
-    if (tid == 0) passTotal = 0;
-    __syncthreads();
-
-    float acc[8][CN];
-    accumulate<DIST, TX, CN, KT, NST>(a.Xt, a.ld, a.d, rowPoint, colPoint, As, Bs, acc);
-    int ty, tx;
-    tile_coords<TX>(tid, ty, tx);
-
-    // epilogue
-    int myPass = 0;
-    int colPass[CN];
-#pragma unroll
-    for (int j = 0; j < CN; ++j) colPass[j] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = ty + 16 * i;
-        const int p = rowPoint[row];
-        unsigned lo = 0, hi = 0;
-#pragma unroll
-        for (int j = 0; j < CN; ++j) {
-            const int col = tx + TX * j;
-            const int q = colPoint[col];
-            const float dist = finish<DIST>(acc[i][j]);
-            const bool pass = p >= 0 && q >= 0 && p != q && dist <= a.eps;
-            if (pass) {
-                if (col < 32) lo |= 1u << col;
-                else hi |= 1u << (col - 32);
-                colPass[j] += 1;
-                ++myPass;
+        for (int i = tid; i < TM; i += NT) {
+            const int64_t q = mbeg + i;
+            if (q < mend) {
+                const int2 mb = a.members[q];
+                rowPoint[i] = mb.x;
+                rowSlot[i] = mb.y;
+            } else {
+                rowPoint[i] = -1;
+                rowSlot[i] = 0;
             }
-            if (a.dists != nullptr && p >= 0 && q >= 0)
-                a.dists[((size_t)p * 2 * a.k + rowSlot[row]) * a.m + ct * TN + col] = dist;
+            smask[2 * i] = 0;
+            smask[2 * i + 1] = 0;
         }
-        if (lo) atomicOr(&smask[2 * row], lo);
-        if (hi) atomicOr(&smask[2 * row + 1], hi);
-    }
+        for (int j = tid; j < TNK; j += NT) {
+            const int c = ct * TN + j;
+            colPoint[j] = c < a.m ? cand[c] : -1;
+            colCount[j] = 0;
+        }
+        if (tid == 0) passTotal = 0;
+        __syncthreads();
+
+        float acc[8][CN];
+        accumulate<DIST, TX, CN, KT, NST>(a.Xt, a.ld, a.d, rowPoint, colPoint, As, Bs, acc);
+        int ty, tx;
+        tile_coords<TX>(tid, ty, tx);
+
+        // epilogue
+        int myPass = 0;
+        int colPass[CN];
 #pragma unroll
-    for (int j = 0; j < CN; ++j)
-        if (colPass[j]) atomicAdd(&colCount[tx + TX * j], colPass[j]);
-    const int wp = warp_sum(myPass);
-    if ((tid & 31) == 0 && wp) atomicAdd(&passTotal, wp);
-    __syncthreads();
-    for (int row = tid; row < TM; row += NT) {
-        const int p = rowPoint[row];
-        if (p >= 0) {
-            const uint64_t w = ((uint64_t)smask[2 * row + 1] << 32) | smask[2 * row];
-            a.masks[((size_t)p * 2 * a.k + rowSlot[row]) * a.W + ct] = w;
+        for (int j = 0; j < CN; ++j) colPass[j] = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = ty + 16 * i;
+            const int p = rowPoint[row];
+            unsigned lo = 0, hi = 0;
+#pragma unroll
+            for (int j = 0; j < CN; ++j) {
+                const int col = tx + TX * j;
+                const int q = colPoint[col];
+                const float dist = finish<DIST>(acc[i][j]);
+                const bool pass = p >= 0 && q >= 0 && p != q && dist <= a.eps;
+                if (pass) {
+                    if (col < 32) lo |= 1u << col;
+                    else hi |= 1u << (col - 32);
+                    colPass[j] += 1;
+                    ++myPass;
+                }
+                if (a.dists != nullptr && p >= 0 && q >= 0)
+                    a.dists[((size_t)p * 2 * a.k + rowSlot[row]) * a.m + ct * TN + col] = dist;
+            }
+            if (lo) atomicOr(&smask[2 * row], lo);
+            if (hi) atomicOr(&smask[2 * row + 1], hi);
         }
+#pragma unroll
+        for (int j = 0; j < CN; ++j)
+            if (colPass[j]) atomicAdd(&colCount[tx + TX * j], colPass[j]);
+        const int wp = warp_sum(myPass);
+        if ((tid & 31) == 0 && wp) atomicAdd(&passTotal, wp);
+        __syncthreads();
+        for (int row = tid; row < TM; row += NT) {
+            const int p = rowPoint[row];
+            if (p >= 0) {
+                const uint64_t w = ((uint64_t)smask[2 * row + 1] << 32) | smask[2 * row];
+                a.masks[((size_t)p * 2 * a.k + rowSlot[row]) * a.W + ct] = w;
+            }
+        }
+        for (int j = tid; j < TNK; j += NT)
+            if (colCount[j]) atomicAdd(a.inRaw + colPoint[j], colCount[j]);
+        if (tid == 0 && passTotal) atomicAdd(a.pairs, (unsigned long long)passTotal);
+        __syncthreads();  // the next tile reuses the shared memory
     }
-    for (int j = tid; j < TNK; j += NT)
-        if (colCount[j]) atomicAdd(a.inRaw + colPoint[j], colCount[j]);
-    if (tid == 0 && passTotal) atomicAdd(a.pairs, (unsigned long long)passTotal);
 }
 
 template <int DIST, int TX, int CN, int KT = TK, int NST = STAGES> int launch_dist_v(const DistArgs& a, cudaStream_t st) {
@@ -142,7 +145,12 @@ template <int DIST, int TX, int CN, int KT = TK, int NST = STAGES> int launch_di
         cudaSuccess)
         return -1;
     if (a.nTiles <= 0) return 0;
-    k_dist<DIST, TX, CN, KT, NST><<<(unsigned)a.nTiles, 16 * TX, sm, st>>>(a);
+    // A CTA per tile, but behind a gate a few per SM that take the tiles in
+    // turn: the gate is nearly always closed, and starting a CTA per tile to
+    // read it takes 83 us at 1M x 784 (2.6 us this way).
+    const int64_t few = (int64_t)sm_count() * 3;
+    const unsigned grid = (unsigned)(a.gate != nullptr && a.nTiles > few ? few : a.nTiles);
+    k_dist<DIST, TX, CN, KT, NST><<<grid, 16 * TX, sm, st>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
