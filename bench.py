@@ -51,11 +51,11 @@ WORKLOADS = {
 # Chi2 mul, add, div, add)
 DIST_FLOPS = {"Cosine": 2, "L2": 3, "L1": 3, "Chi2": 4, "JS": 8}
 FP32_PEAK_TFLOPS = 152 * 128 * 2 * 2.070e9 / 1e12  # nominal FP32 CUDA-core peak at max SM clock
-# DRAM bytes (read + write) of one k_dist<Cosine> launch on the 1M x 784
+# DRAM bytes (read + write) of one k_dist_pair<Cosine> launch on the 1M x 784
 # workload, from a one-pass ncu capture of
-# `python bench.py --single-fit 1000000 --precision 0` (profiles/k_dist_fp32_cfg2.md):
-# 23.29 GB read + 0.370 GB written (tiles run in point-chunk order).
-K_DIST_TRAFFIC_1M = 23.29e9 + 0.370e9
+# `python bench.py --single-fit 1000000 --precision 0` (profiles/k_dist_pair_fp32_cfg2.md):
+# 22.97 GB read + 0.367 GB written (tiles run in point-chunk order).
+K_DIST_TRAFFIC_1M = 22.97e9 + 0.367e9
 # One CPU fit of the whole 1M x 784 config-2 workload (the reference arm's code,
 # all 16 host cores of the GPU machine): `python bench.py --impl reference
 # --cpu-full-fit`, recorded in profiles/cpu_full_fit_cfg2_1Mx784.md (23 minutes,
@@ -495,7 +495,7 @@ def _cpu_sng(cfg, n_sample=20000):
 def run_sng(args, local, X, cfg, cpu=True):
     """sngDBSCAN on the headline data (n x d resident in HBM): one step =
     one fit_sngDbscan (transform, sample, dense distance block, degrees,
-    union-find labels).  Dominant kernel: k_sng_block, n x (sampled points) x d."""
+    union-find labels).  Dominant kernel: k_sng_pair, n x (sampled points) x d."""
     import numpy as np
     import torch
     from sdbscan_gb300 import capi
@@ -557,7 +557,7 @@ def run_sng(args, local, X, cfg, cpu=True):
            "config": {"samplingProb": SNG_PROB, "random_seed": SNG_SEED, "eps": cfg["eps"], "minPts": cfg["minPts"],
                       "draws_per_point": int(-(-n * SNG_PROB // 1)), "distinct_sampled": c["sng_sampled"],
                       "extra_draws": c["sng_extra"]},
-           "roofline": {"bound": "fp32", "kernel": f"k_sng_block<{cfg['distance']}>", "achieved": achieved,
+           "roofline": {"bound": "fp32", "kernel": f"k_sng_pair<{cfg['distance']}>", "achieved": achieved,
                         "peak": FP32_PEAK_TFLOPS, "unit": "TFLOP/s", "frac": achieved / FP32_PEAK_TFLOPS,
                         "traffic": None, "flops_per_launch": flops, "kernel_ms": stages["distances"],
                         "peak_source": "nominal FP32 CUDA-core peak (152 SMs x 128 lanes x 2 flop x 2.07 GHz)"},
@@ -705,7 +705,7 @@ def run_ours(args, cfg):
         batched = run_batched(args, local, cpu=ws == 1 and not args.no_cpu)
     if rank != 0:
         return 0
-    # dominant kernel: the distance stage (one k_dist launch per fit)
+    # dominant kernel: the distance stage (one k_dist_pair launch per fit)
     dist_ms = stage_sum["distances"] / args.steps
     flops = float(DIST_FLOPS[cfg["distance"]]) * (2 * cfg["topK"] * cfg["topM"]) * d * n
     achieved = flops / (dist_ms / 1e3) / 1e12
@@ -713,7 +713,7 @@ def run_ours(args, cfg):
     traffic = K_DIST_TRAFFIC_1M if cfg["workload"].startswith("cfg2") else None
     alg_bytes = n * d * 4 + 2 * cfg["n_proj"] * cfg["topM"] * d * 4  # rows of X + candidate rows, once each
     sgemm = _sgemm_tflops(f"cuda:{local}")
-    roofline = {"bound": "fp32", "kernel": f"k_dist<{cfg['distance']}>", "achieved": achieved, "peak": FP32_PEAK_TFLOPS,
+    roofline = {"bound": "fp32", "kernel": f"k_dist_pair<{cfg['distance']}>", "achieved": achieved, "peak": FP32_PEAK_TFLOPS,
                 "unit": "TFLOP/s", "frac": achieved / FP32_PEAK_TFLOPS, "traffic": traffic,
                 "measured_fp32_gemm": {"tflops": sgemm, "frac": achieved / sgemm,
                                        "source": "cuBLAS FP32 GEMM 8192^3, TF32 off, timed in this run"},
@@ -721,7 +721,7 @@ def run_ours(args, cfg):
                               "pipe, not by HBM or the tensor cores; the BF16 leg carries the tensor roofline",
                 "peak_source": "nominal FP32 CUDA-core peak (152 SMs x 128 lanes x 2 flop x 2.07 GHz); "
                                "MEASURED_PEAKS.json has no FP32 figure",
-                "traffic_source": "ncu dram__bytes_read+write of one k_dist launch on this workload",
+                "traffic_source": "ncu dram__bytes_read+write of one k_dist_pair launch on this workload",
                 "hbm_view": {"algorithmic_bytes": alg_bytes, "achieved_gbs": alg_bytes / (dist_ms / 1e3) / 1e9,
                              "measured_traffic_gbs": traffic / (dist_ms / 1e3) / 1e9 if traffic else None,
                              "peak_gbs": hbm_peak, "peak_source": src},
