@@ -55,11 +55,13 @@ __device__ __forceinline__ bool tile_of(const ClusterArgs& a, int64_t b, Tile& t
 // its own the tile pass would send some twenty unites per point at the same few
 // roots, all at once; after the rounds it finds almost nothing but equal roots
 // (1M x 784: union 1827 us without, 291 + 263 for the rounds; hooking only the
-// own root left 955, walking to the members' roots first 613).
+// own root left 955, walking to the members' roots first 613).  In an eps sweep's
+// later rounds the tile pass sees the new edges only, those hooked by among them.
 __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !a.core[p] || (a.carry && a.coreEps[p] != a.round)) return;
-    RootSpan span(round_root(a.parent, p, a.n));
+    const bool carried = a.carry && a.round > 0;
+    RootSpan span(round_root(a.parent, p, a.n, carried));
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int j = (slot0 + t) % (2 * a.k);
@@ -69,7 +71,7 @@ __global__ void __launch_bounds__(256) k_hook(ClusterArgs a, int slot0) {
         const int32_t* cand = a.topM + (size_t)__ldg(a.topK + at) * 2 * a.m + (j >= a.k ? a.m : 0);
         for (int c = 0; c < 2 && bits; ++c, bits &= bits - 1) {
             const int q = __ldg(cand + __ffsll((long long)bits) - 1);
-            if (a.core[q]) span.see(round_root(a.parent, q, a.n));
+            if (a.core[q]) span.see(round_root(a.parent, q, a.n, carried));
         }
     }
     span.hook(a.parent);
