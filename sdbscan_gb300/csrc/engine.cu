@@ -204,19 +204,22 @@ void sdb_engine::host_random(int seedUsed) {
 // the fit pipeline
 // ---------------------------------------------------------------------------
 sdb_status sdb_engine::fit(const float* X, bool xOnDevice, float eps, int minPts, bool optics, const SweepSpec* sw) {
-    sdb_status s = fit_once(X, xOnDevice, eps, minPts, optics, sw);
-    // out of memory with the packed tile's candidate copy: once more without it
+    sdb_status s = fit_once(X, xOnDevice, eps, minPts, optics, sw, true);
+    // out of memory with the packed tile's candidate copy (this fit's or an
+    // earlier one's): once more without it, and without the distances that
+    // another kind of fit left.  The next fit tries the copy again: it may be
+    // smaller, or the memory free by then.
     if (s == SDB_ERR_NOMEM && candT.ptr != nullptr && !(sw != nullptr && sw->capture)) {
         cudaStreamSynchronize(stream);
         release(candT);
-        noCandCopy = true;
-        s = fit_once(X, xOnDevice, eps, minPts, optics, sw);
+        release(dists);
+        s = fit_once(X, xOnDevice, eps, minPts, optics, sw, false);
     }
     return s;
 }
 
 sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int minPts, bool optics,
-                                const SweepSpec* sw) {
+                                const SweepSpec* sw, bool candCopy) {
     if (!paramsSet) return fail(SDB_ERR_STATE, "set_params must be called before a fit");
     const bool sweep = sw != nullptr, capture = sw != nullptr && sw->capture;
     if (sweep && (optics || sw->nEps < 1 || !sw->eps || !sw->labelsDev || !sw->nclDev))
@@ -262,8 +265,10 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     // 4K x 128, 20 members: 82 against 92; 50K x 128, 244: 232 against 309).
     const bool wantPair = distVariant == 3 || (distVariant == 0 && (int64_t)n * k >= (int64_t)kMinCandMembers * D);
     const int pairCols = screen || !wantPair ? 0 : pair_tile_cols(p.distance, m);
-    const bool pairTiles = pairCols > 0 && !noCandCopy && pair_cand_bytes(pairCols, D, m, ld) <= kMaxCandBytes &&
-                           ensure(candT, pair_cand_bytes(pairCols, D, m, ld));
+    // (A capture allocates nothing: it takes the tile of the run that sized it.)
+    const size_t candBytes = pairCols > 0 ? pair_cand_bytes(pairCols, D, m, ld) : 0;
+    const bool pairTiles = pairCols > 0 && candCopy && candBytes <= kMaxCandBytes &&
+                           (capture ? candT.bytes >= candBytes : ensure(candT, candBytes));
     const int TMr = pairTiles ? pair_tile_rows(pairCols) : dist_tile_rows();
     const int CT = pairTiles ? pairCols : dist_tile_cols();
     const int nct = (m + CT - 1) / CT, W = nct;

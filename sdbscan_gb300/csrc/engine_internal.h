@@ -106,7 +106,6 @@ struct sdb_engine {
     int64_t fallbacks = 0;  // BF16 screening fits redone on the plain path
     int sngColsLast = 0, sngExtraLast = 0;  // sampled columns and extra draws of the last sng fit
     int distVariant = 0;    // plain distance tile shape (DistArgs::variant), set by the batch's autotuner
-    bool noCandCopy = false;  // the packed distance tile's candidate copy did not fit in memory
     int sngSampling = 0;    // sngDbscan sample: 0 = by seed (shared when >= 0, blocks when < 0), 1 = shared, 2 = blocks
     // test and diagnostic limits (sdb_set_debug_limits), 0 = off
     long long dbgStallSpins = 0;  // each tensor-core / persistent distance kernel takes its failure path once
@@ -125,7 +124,9 @@ struct sdb_engine {
     void host_random(int seed);
     sdb_status fit(const float* X, bool xOnDevice, float eps, int minPts, bool optics,
                    const SweepSpec* sw = nullptr);
-    sdb_status fit_once(const float* X, bool xOnDevice, float eps, int minPts, bool optics, const SweepSpec* sw);
+    // candCopy: the packed distance tile's candidate copy may be made
+    sdb_status fit_once(const float* X, bool xOnDevice, float eps, int minPts, bool optics, const SweepSpec* sw,
+                        bool candCopy);
     sdb_status check_flags();
     sdb_status optics_stage(const sdb::CoreArgs& ca, int& launches);
     sdb_status optics_order(int64_t total);
@@ -134,10 +135,10 @@ struct sdb_engine {
     sdb_status fit_sng(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
                        int32_t* labelsOut = nullptr, int32_t* nclOut = nullptr);
     sdb_status fit_sng_once(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
-                            int32_t* labelsOut, int32_t* nclOut);
+                            int32_t* labelsOut, int32_t* nclOut, bool colCopy);
     // sngDbscan with independent samples per block of points (k_sng_blocks.cu)
     sdb_status fit_sng_blocks(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts, bool optics,
-                              int32_t* labelsOut, int32_t* nclOut);
+                              int32_t* labelsOut, int32_t* nclOut, bool colCopy);
 
     static float* f32(DevBuf& b) { return static_cast<float*>(b.ptr); }
     static int32_t* i32(DevBuf& b) { return static_cast<int32_t*>(b.ptr); }

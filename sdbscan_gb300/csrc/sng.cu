@@ -101,20 +101,20 @@ const char* dist_label(int d) {
 
 sdb_status sdb_engine::fit_sng(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts,
                                bool optics, int32_t* labelsOut, int32_t* nclOut) {
-    sdb_status s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut);
-    // out of memory with the packed tile's column copy: once more without it
+    sdb_status s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut, true);
+    // out of memory with the packed tile's column copy: once more without it (as
+    // sdb_engine::fit)
     if (s == SDB_ERR_NOMEM && candT.ptr != nullptr) {
         cudaStreamSynchronize(stream);
         release(candT);
         release(dists);
-        noCandCopy = true;
-        s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut);
+        s = fit_sng_once(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut, false);
     }
     return s;
 }
 
 sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts,
-                                    bool optics, int32_t* labelsOut, int32_t* nclOut) {
+                                    bool optics, int32_t* labelsOut, int32_t* nclOut, bool colCopy) {
     if (!paramsSet && !sngParamsSet) return fail(SDB_ERR_STATE, "set_sngParams must be called before a fit");
     if (X == nullptr) return fail(SDB_ERR_ARG, "X is null");
     if (epsList == nullptr || nEps < 1 || (optics && nEps != 1)) return fail(SDB_ERR_ARG, "invalid eps list");
@@ -137,7 +137,7 @@ sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float*
     // std::random_device, so blocks unless a shared sample is asked for)
     if (optics ? sngSampling != 1
                : p.samplingProb < 1.0 && (sngSampling == 2 || (sngSampling == 0 && p.random_seed < 0)))
-        return fit_sng_blocks(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut);
+        return fit_sng_blocks(X, xOnDevice, epsList, nEps, minPts, optics, labelsOut, nclOut, colCopy);
 
     SngSample smp;
     sng_sample(n, p.samplingProb, (unsigned)seedUsed, optics, smp);
@@ -160,7 +160,7 @@ sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float*
     // only if the screening fails)
     const bool screen = !optics && p.precision == SDB_PREC_BF16 && p.distance == SDB_COSINE && nU > 0;
     const size_t copyBytes = optics || screen ? 0 : sng_pair_bytes(p.distance, nU, ld);
-    const bool packed = copyBytes > 0 && !noCandCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
+    const bool packed = copyBytes > 0 && colCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
                         (p.distance != SDB_CHI2 || ensure(smallEntry, n));
     if (!optics)
         ok &= ensure(sngMask, sizeof(uint64_t) * std::max<size_t>(1, (size_t)nct * n)) &&
@@ -378,7 +378,7 @@ sdb_status sdb_engine::fit_sng_once(const float* X, bool xOnDevice, const float*
 // (k_sng_blocks.cu): transform, then per eps the pass words, degrees and core
 // flags, the union-find over the core-core passes, border minima and labels.
 sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const float* epsList, int nEps, int minPts,
-                                      bool optics, int32_t* labelsOut, int32_t* nclOut) {
+                                      bool optics, int32_t* labelsOut, int32_t* nclOut, bool colCopy) {
     const sdb_params& p = prm;
     const int BR = sng_block_rows();
     // draws per point: ceil(1.0 n prob) in double (src/sDbscan.cpp:432), for
@@ -402,7 +402,7 @@ sdb_status sdb_engine::fit_sng_blocks(const float* X, bool xOnDevice, const floa
     // 784, 500 draws, pass and copy: 0.87 and 0.99), and for sngOptics always,
     // which keeps its distances
     const size_t copyBytes = S > 0 && (optics || S >= kMinPackedDraws) ? sng_pair_bytes(p.distance, n, ld) : 0;
-    const bool packed = copyBytes > 0 && !noCandCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
+    const bool packed = copyBytes > 0 && colCopy && copyBytes <= kMaxCandBytes && ensure(candT, copyBytes) &&
                         (p.distance != SDB_CHI2 || ensure(smallEntry, n));
     // sngOptics keeps the pass's distances for its emitting pass
     const size_t distBytes = sizeof(float) * (size_t)nb * BR * (size_t)std::max<int64_t>(S, 0);
