@@ -364,9 +364,11 @@ struct CsrArgs {
     const int32_t* newId;  // n
     int64_t* edgeOff;      // n + 1 out
     uint2* edges;          // (newId of the neighbour, key of max(core distance, distance)) out
+    int64_t begin, end;    // entries of the regrouped lists to write, to edges[0] on
 };
 int launch_csr_starts(const CsrArgs& a, cudaStream_t st);
-int launch_csr_edges(const CsrArgs& a, int64_t* scanTmp, cudaStream_t st);
+int launch_csr_offsets(const CsrArgs& a, int64_t* scanTmp, cudaStream_t st);
+int launch_csr_edges(const CsrArgs& a, cudaStream_t st);
 
 // sngDbscan / sngOptics (src/sDbscan.cpp:416-504, :1484-1583) over one
 // shared sample of columns: every point is a row, every distinct sampled

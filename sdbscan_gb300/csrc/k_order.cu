@@ -71,15 +71,17 @@ __global__ void k_csr_lengths(CsrArgs a) {
     if (p < a.n) a.edgeOff[a.newId[p]] = a.core[p] ? a.off[p + 1] - a.off[p] : 0;
 }
 
-// A warp per core point: its list at the point's new place.  A neighbour of
-// another flood becomes the point itself, which is done when its list is read.
+// A warp per core point: its list at the point's new place, as far as that lies
+// in [begin, end).  A neighbour of another flood becomes the point itself, which
+// is done when its list is read.
 __global__ void __launch_bounds__(256) k_csr_edges(CsrArgs a) {
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= a.n || !a.core[p]) return;
     const int me = a.newId[p], s = a.start[p];
     const float cd = a.coreDist[p];
-    const int64_t e0 = a.off[p], e1 = a.off[p + 1], o = a.edgeOff[me] - e0;
-    for (int64_t t = e0 + lane_id(); t < e1; t += 32) {
+    const int64_t e0 = a.off[p], o = a.edgeOff[me] - e0 - a.begin;  // entry t goes to edges[o + t]
+    const int64_t t0 = max(e0, -o), t1 = min(a.off[p + 1], a.end - a.begin - o);
+    for (int64_t t = t0 + lane_id(); t < t1; t += 32) {
         const int q = __ldg(a.idx + t);
         const int to = __ldg(a.start + q) == s ? __ldg(a.newId + q) : me;
         a.edges[o + t] = make_uint2((uint32_t)to, key_of(fmaxf(cd, __ldg(a.dist + t))));
@@ -108,13 +110,16 @@ int launch_csr_starts(const CsrArgs& a, cudaStream_t st) {
     return cudaPeekAtLastError() == cudaSuccess ? launches + 3 : -1;
 }
 
-int launch_csr_edges(const CsrArgs& a, int64_t* scanTmp, cudaStream_t st) {
+int launch_csr_offsets(const CsrArgs& a, int64_t* scanTmp, cudaStream_t st) {
     k_csr_lengths<<<(a.n + 255) / 256, 256, 0, st>>>(a);
     if (cudaPeekAtLastError() != cudaSuccess) return -1;
     const int r = launch_scan_i64(a.edgeOff, a.edgeOff, (size_t)a.n + 1, scanTmp, st);
-    if (r < 0) return -1;
+    return r < 0 ? -1 : r + 1;
+}
+
+int launch_csr_edges(const CsrArgs& a, cudaStream_t st) {
     k_csr_edges<<<(a.n + 7) / 8, 256, 0, st>>>(a);
-    return cudaPeekAtLastError() == cudaSuccess ? r + 2 : -1;
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
 }  // namespace sdb

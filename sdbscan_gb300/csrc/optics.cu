@@ -37,6 +37,8 @@ struct Edge {
     uint32_t to, key;  // neighbour's number, order-preserving key of max(core distance, distance)
 };
 
+constexpr int64_t kMinPiece = 4096;  // entries of the smallest piece that the lists come over in
+
 constexpr uint32_t kDone = 0, kUnreached = 0xffffffffu;  // no float has these keys
 
 // The inverse of key_of (common.cuh).
@@ -160,19 +162,25 @@ sdb_status sdb_engine::optics_stage(const CoreArgs& ca, int& launches) {
 sdb_status sdb_engine::optics_order(int64_t total) {
     cudaStream_t st = stream;
     cudaError_t e = cudaSuccess;
-    if (!ensure(parent, sizeof(int32_t) * n) || !ensure(border, sizeof(int32_t) * n) ||
-        !ensure(floodStart, sizeof(int32_t) * n) || !ensure(newId, sizeof(int32_t) * n) ||
-        !ensure(edgeOff, sizeof(int64_t) * (n + 1)))
-        return SDB_ERR_NOMEM;
-    const size_t edgeBytes = sizeof(Edge) * std::max<int64_t>(total, 1);
-    if (!ensure(edges, edgeBytes)) {
-        // the lists are made: what only the distance stage reads makes room
-        // (the distances alone are n x 2k x m floats)
+    // The lists are made: where the ordering's buffers do not fit, those that
+    // only the stages before read make room (the distances are n x 2k x m
+    // floats, sngOptics' tables 16 bytes an entry and more).  Where the regrouped
+    // lists do not fit even then, they come over in pieces.
+    auto points = [&]() {
+        return ensure(parent, sizeof(int32_t) * n) && ensure(border, sizeof(int32_t) * n) &&
+               ensure(floodStart, sizeof(int32_t) * n) && ensure(newId, sizeof(int32_t) * n) &&
+               ensure(edgeOff, sizeof(int64_t) * (n + 1));
+    };
+    int64_t piece = std::max<int64_t>(total, 1);
+    if (!points() || !ensure(edges, sizeof(Edge) * piece)) {
         e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cuda_fail(e, "neighbour lists");
-        release(dists);
-        release(candT);
-        if (!ensure(edges, edgeBytes)) return SDB_ERR_NOMEM;
+        for (DevBuf* b : {&dists, &candT, &hashIdB, &hashDistB, &sngWords}) release(*b);
+        if (!points()) return SDB_ERR_NOMEM;
+        while (!ensure(edges, sizeof(Edge) * piece)) {
+            if (piece <= kMinPiece) return SDB_ERR_NOMEM;
+            piece = std::max(kMinPiece, (piece + 1) / 2);
+        }
     }
     CsrArgs a{};
     a.n = n;
@@ -221,12 +229,21 @@ sdb_status sdb_engine::optics_order(int64_t total) {
     }
     e = cudaMemcpyAsync(newId.ptr, hNew, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(e, "flood numbers");
-    if (launch_csr_edges(a, i64(scanTmp), st) < 0) return fail(SDB_ERR_CUDA, "flood list launch failed");
+    a.end = piece;
+    if (launch_csr_offsets(a, i64(scanTmp), st) < 0 || launch_csr_edges(a, st) < 0)
+        return fail(SDB_ERR_CUDA, "flood list launch failed");
     e = cudaMemcpyAsync(hOff, edgeOff.ptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     const int64_t kept = e == cudaSuccess ? hOff[n] : 0;
-    if (e == cudaSuccess && kept)
-        e = cudaMemcpyAsync(hEdges, edges.ptr, sizeof(Edge) * kept, cudaMemcpyDeviceToHost, st);
+    for (int64_t at = 0; e == cudaSuccess && at < kept; at += piece) {
+        if (at > 0) {
+            a.begin = at;
+            a.end = at + piece;
+            if (launch_csr_edges(a, st) < 0) return fail(SDB_ERR_CUDA, "flood list launch failed");
+        }
+        e = cudaMemcpyAsync(hEdges + at, edges.ptr, sizeof(Edge) * std::min(piece, kept - at), cudaMemcpyDeviceToHost,
+                            st);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "neighbour list download");
 
