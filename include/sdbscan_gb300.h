@@ -309,7 +309,7 @@ const char* sdb_batch_last_error(sdb_batch* b);
  * SDB_ERR_ARG.  When n_proj is a multiple of 4 the rows are read as 16-byte
  * vectors, so proj_device must then be 16-byte aligned (SDB_ERR_ARG
  * otherwise; an offset view into a larger buffer may not be).
- * Scratch is one fixed __device__ array (about 10 MiB) held by every GPU that
+ * Scratch is one fixed __device__ array (about 12 MiB) held by every GPU that
  * loads this library until it is unloaded.  With CUDA's lazy module loading
  * (the default) the array is reserved on a device by the first call there,
  * which also looks up its device address: make that first call before the

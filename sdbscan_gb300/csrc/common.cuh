@@ -135,6 +135,7 @@ struct TopMArgs {
     const float* P;
     int n, nproj, m;
     const uint32_t* chunkExt;  // ProjectArgs::chunkExt
+    const uint2* chunkKeys;    // or, in its place, key_of of the chunk's max v and max -v
     int G;
     float* thrMax;       // nproj
     float* thrMin;       // nproj

@@ -5,7 +5,7 @@
 // Exact without a per-vector heap over n:
 //  1. The projection kernel leaves, for every chunk of points, the maximum
 //     and minimum projection onto each vector (as BF16 rounded away from the
-//     extreme, so still bounds of attained values).  The m-th largest of the chunk
+//     extreme, so still bounds of attained values; 32-bit keys where the caller made them).  The m-th largest of the chunk
 //     maxima is a value attained by m different points, so it is a lower
 //     bound T on the true m-th largest value (k_thresholds).
 //  2. One pass over the projections appends every (value, point) with value
@@ -53,8 +53,8 @@ __host__ __device__ inline int pow2_ceil(int x) {
 // T of every list (r, side): the m-th largest chunk extreme, 0 with fewer than
 // m of them.  A CTA takes `cols` neighbouring vectors (32-byte row segments with
 // 8), folds `group` chunks into one (their maximum is attained too) and keeps
-// the results' 16-bit order-preserving keys in shared memory; a warp then finds
-// a list's m-th largest key by bisection, counting 16 times.
+// the results' order-preserving keys in shared memory; a warp then finds a list's
+// m-th largest key by bisection, counting once per bit of a key.
 // The chunks folded into one are ng apart, each layer of ng rotated against the
 // one before: points that arrive cluster after cluster, or in several such
 // runs, keep about as many chunks of their own as without folding.  (Folding
@@ -67,33 +67,56 @@ __host__ __device__ inline int pow2_ceil(int x) {
 // above 44K, D = 1024 (45 at 2K); this takes 30 (14), about half of it the
 // bisections.
 constexpr int kThrThreads = 512;
-__device__ __forceinline__ uint32_t key16(uint32_t b) { return (b & 0x8000u) ? ~b & 0xffffu : b | 0x8000u; }
+// A chunk's extremes (TopMArgs::chunkExt, chunkKeys) as the keys of both sides.
+struct Keys16 {
+    static constexpr int kBits = 16;
+    typedef uint32_t Pair;  // close side in the low half
+    static __device__ __forceinline__ Pair none() { return 0xffffffffu; }  // as loaded: the least keys
+    static __device__ __forceinline__ Pair load(const TopMArgs& a, size_t at) { return __ldg(a.chunkExt + at); }
+    static __device__ __forceinline__ Pair keys(Pair b) {  // a set sign bit flips its half, else that bit alone flips
+        return b ^ (((b >> 15) & 0x00010001u) * 0x7fffu | 0x80008000u);
+    }
+    static __device__ __forceinline__ Pair larger(Pair x, Pair y) {
+        Pair z;
+        asm("max.u16x2 %0, %1, %2;" : "=r"(z) : "r"(x), "r"(y));
+        return z;
+    }
+    static __device__ __forceinline__ uint32_t of(Pair x, int side) { return side ? x >> 16 : x & 0xffffu; }
+};
+struct Keys32 {
+    static constexpr int kBits = 32;
+    typedef uint2 Pair;
+    static __device__ __forceinline__ Pair none() { return make_uint2(0u, 0u); }
+    static __device__ __forceinline__ Pair load(const TopMArgs& a, size_t at) { return __ldg(a.chunkKeys + at); }
+    static __device__ __forceinline__ Pair keys(Pair b) { return b; }
+    static __device__ __forceinline__ Pair larger(Pair x, Pair y) { return make_uint2(max(x.x, y.x), max(x.y, y.y)); }
+    static __device__ __forceinline__ uint32_t of(Pair x, int side) { return side ? x.y : x.x; }
+};
 
+template <class K>
 __global__ void __launch_bounds__(kThrThreads) k_thresholds(TopMArgs a, int cols, int group, int ng) {
-    extern __shared__ uint32_t keys[];  // ng x stride: (max key << 16) | min side's key
+    extern __shared__ __align__(8) unsigned char thrShm[];
+    typename K::Pair* keys = reinterpret_cast<typename K::Pair*>(thrShm);  // ng x stride
     const int stride = cols | 1;
     const int c = threadIdx.x & (cols - 1), r = blockIdx.x * cols + c, step = kThrThreads / cols;
     if (r < a.nproj) {
         const int turn = ng / 8 * 5;
         for (int q = threadIdx.x / cols; q < ng; q += step) {
-            uint32_t hi = 0, lo = 0;
+            typename K::Pair most = K::keys(K::none());
             int x = q;
-            for (int j = 0; j < group; j += 8) {  // eight loads in flight (no chunk: the least key)
-                uint32_t e[8];
+            for (int j = 0; j < group; j += 8) {  // eight loads in flight
+                typename K::Pair e[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int g = (j + u) * ng + x;
-                    e[u] = g < a.G ? __ldg(a.chunkExt + (size_t)g * a.nproj + r) : 0xffffffffu;
+                    e[u] = g < a.G ? K::load(a, (size_t)g * a.nproj + r) : K::none();
                     x += turn;
                     if (x >= ng) x -= ng;
                 }
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    hi = max(hi, key16(e[u] & 0xffffu));
-                    lo = max(lo, key16(e[u] >> 16));
-                }
+                for (int u = 0; u < 8; ++u) most = K::larger(most, K::keys(e[u]));
             }
-            keys[q * stride + c] = (hi << 16) | lo;
+            keys[q * stride + c] = most;
         }
     }
     __syncthreads();
@@ -103,17 +126,14 @@ __global__ void __launch_bounds__(kThrThreads) k_thresholds(TopMArgs a, int cols
         if (rr >= a.nproj) break;
         uint32_t t = 0;
         if (ng >= a.m) {
-            for (int bit = 15; bit >= 0; --bit) {
+            for (int bit = K::kBits - 1; bit >= 0; --bit) {
                 const uint32_t at = t | (1u << bit);
                 int cnt = 0;
 #pragma unroll 8
-                for (int q = lane; q < ng; q += 32) {
-                    const uint32_t k = keys[q * stride + col];
-                    cnt += (side ? k & 0xffffu : k >> 16) >= at;
-                }
+                for (int q = lane; q < ng; q += 32) cnt += K::of(keys[q * stride + col], side) >= at;
                 if (warp_sum(cnt) >= a.m) t = at;
             }
-            t <<= 16;  // the smallest 32-bit key with these high bits
+            t <<= 32 - K::kBits;  // the smallest 32-bit key with these high bits
         }
         if (lane == 0) (side ? a.thrMin : a.thrMax)[rr] = __uint_as_float(t);  // raw key bits
     }
@@ -358,18 +378,22 @@ __global__ void k_select(TopMArgs a) {
 
 }  // namespace
 
-int launch_topm_thresholds(const TopMArgs& a, cudaStream_t st) {
+template <class K> static int launch_thresholds(const TopMArgs& a, cudaStream_t st) {
     // 912 groups or 4m: enough that the m-th largest is close to the m-th value
     const int group = std::max(1, a.G / std::max(912, 4 * a.m));
     const int ng = (a.G + group - 1) / group;
     int cols = 8;
-    while (cols > 1 && sizeof(uint32_t) * (size_t)ng * (cols | 1) > 100 * 1024) cols >>= 1;
-    const size_t sm = sizeof(uint32_t) * (size_t)ng * (cols | 1);
+    while (cols > 1 && sizeof(typename K::Pair) * (size_t)ng * (cols | 1) > 100 * 1024) cols >>= 1;
+    const size_t sm = sizeof(typename K::Pair) * (size_t)ng * (cols | 1);
     if (sm > 48 * 1024 &&
-        cudaFuncSetAttribute(k_thresholds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+        cudaFuncSetAttribute(k_thresholds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
         return -1;
-    k_thresholds<<<(a.nproj + cols - 1) / cols, kThrThreads, sm, st>>>(a, cols, group, ng);
+    k_thresholds<K><<<(a.nproj + cols - 1) / cols, kThrThreads, sm, st>>>(a, cols, group, ng);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+
+int launch_topm_thresholds(const TopMArgs& a, cudaStream_t st) {
+    return a.chunkKeys != nullptr ? launch_thresholds<Keys32>(a, st) : launch_thresholds<Keys16>(a, st);
 }
 
 int launch_topm_collect(const TopMArgs& a, cudaStream_t st) {
