@@ -108,7 +108,7 @@ struct ProjectArgs {
     double ln4;              // JS: log(4.0) as the host computes it
     uint16_t* Xb;            // Cosine, fhtDim <= 2048: BF16 copy of Xt (n x ldb, zero padded), or null
     int ldb;                 // its row stride, <= fhtDim
-    uint8_t* small;          // Chi2: n flags out, the transformed row has an entry in (0, 2^-50); or null
+    uint8_t* small;          // Chi2: n flags out, the transformed row has an entry in (0, kChi2Small); or null
 };
 int launch_project(const ProjectArgs& a, cudaStream_t st);
 // Blocks in one full wave of k_project (six blocks per SM; each walks its
@@ -215,7 +215,7 @@ struct DistArgs {
     int nproj, m, k, W;   // W = 64-bit mask words per (point, slot), one per candidate tile
     int nct;              // candidate tiles per list (= W)
     int TM, CT;           // member rows and candidate columns per tile: bit j of word w is column CT w + j
-    const uint8_t* small; // Chi2: per point, a positive entry below 2^-50 (ProjectArgs::small)
+    const uint8_t* small; // Chi2: per point, an entry in (0, kChi2Small) (ProjectArgs::small)
     float* cand;          // packed tile: the lists' candidate rows, dimension-major (launch_cand_tiles), or null
     float eps;
     float epsLo;          // eps sweeps: k_masks_from_dists keeps epsLo < d <= eps

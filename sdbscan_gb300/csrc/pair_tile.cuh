@@ -26,68 +26,18 @@
 #pragma once
 
 #include "dist_tile.cuh"
+#include "f32x2.cuh"
+#include "quotients.cuh"
 
 namespace sdb {
 namespace ptile {
-
-typedef unsigned long long u64;
 
 constexpr int kThreads = 128;        // four warps
 constexpr int KT = 32;               // dimensions per stage
 constexpr int LDA = KT + 4;          // row stride of the staged rows (conflict-free 16-byte reads)
 constexpr int NST = 2;               // stages
 
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
-// Chi2 terms x y / (x + y) of two pairs, correctly rounded, from a = -x and
-// b = -y: n = a b, D = a + b = -(x + y).  A reciprocal estimate, one Newton
-// step on it and one residual correction of the quotient (Markstein, IBM J.
-// Res. Dev. 34 (1990) 111): every operation but the estimate is packed.  Equal
-// to __fdiv_rn for all 2^46 pairs of significands (run through on the GPU), so
-// for all operands in range, and the range is kept by chi2_small: n is 0 or
-// >= 2^-100, which keeps the residual exact.  Where x + y < 2^-100, n is 0 and
-// so is the term, as long as the clamped D keeps the reciprocal finite.
-// The compiled division takes about 36 issue slots a term with its range
-// checks, this takes 6: 60K x 512, k = 10, m = 50, 27.7 -> 9.6 ms.  Bound: the
-// reciprocal unit (16 a cycle and SM, 6.2 ms) beside 8 FMA-pipe slots a term.
-constexpr float kChi2Small = 0x1p-50f;   // entries of (0, this) send a tile to the general term
-__device__ __forceinline__ u64 chi2_terms(u64 a, u64 b) {
-    const u64 n = mul2(a, b);
-    float d0, d1, y0, y1;
-    unpack2(add2(a, b), d0, d1);
-    d0 = fminf(d0, -0x1p-100f);
-    d1 = fminf(d1, -0x1p-100f);
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(-d0));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(-d1));
-    const u64 D = pack2(d0, d1), y = pack2(y0, y1);
-    const u64 z = fma2(fma2(D, y, pack2(1.0f, 1.0f)), y, y);  // 1 / (x + y)
-    const u64 q = mul2(n, z);
-    return fma2(fma2(D, q, n), z, q);
-}
-
-// The general Chi2 term (any entries), a tile's slow form.
+// The general Chi2 term, the form of tiles with an entry in (0, kChi2Small).
 constexpr int DIST_CHI2_ANY = 5;
 
 // One dimension of two pairs: a the row's value in both halves (negated for
