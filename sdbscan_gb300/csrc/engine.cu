@@ -258,11 +258,11 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
     const int ldb = (d + 63) / 64 * 64;
     // the distance tiles: the packed tile where the distance has one (and no
     // other shape is asked for), else 128 x 64.  It reads a copy of the lists'
-    // candidate rows; past kMaxCandBytes (wide data and many vectors) that
-    // copy costs more memory than a list's few tiles are worth, and below
-    // kMinCandMembers members per list it takes longer than the tiles save
-    // (2K x 64, k = 5, D = 1024, 10 members: 47 us with the copy, 43 without;
-    // 4K x 128, 20 members: 82 against 92; 50K x 128, 244: 232 against 309).
+    // candidate rows, kMaxCandBytes at most (a bound on memory, not on speed),
+    // and below kMinCandMembers members per list the copy takes longer than the
+    // tiles save (2K x 64, k = 5, D = 1024, 10 members: 47 us with the copy, 43
+    // without; 4K x 128, 20 members: 82 against 92; 50K x 128, 244: 232 against
+    // 309).
     const bool wantPair = distVariant == 3 || (distVariant == 0 && (int64_t)n * k >= (int64_t)kMinCandMembers * D);
     const int pairCols = screen || !wantPair ? 0 : pair_tile_cols(p.distance, m);
     // (A capture allocates nothing: it takes the tile of the run that sized it.)
@@ -418,7 +418,7 @@ sdb_status sdb_engine::fit_once(const float* X, bool xOnDevice, float eps, int m
         // part of the points only, about 0.08 ms a segment, and the link brings
         // 190 GB/s.  Projection stage with 16 segments against this rule: 40K x
         // 256 (41 MB) 1.58 and 0.50 ms, 70K x 784 (220 MB) 4.43 and 1.79, 200K x
-        // 784 (627 MB) 7.86 and 4.75; 1M x 784 keeps twelve.
+        // 784 (627 MB) 7.86 and 4.75; 1M x 784 (3.1 GB) runs in eleven.
         const size_t xBytes = sizeof(float) * (size_t)n * d;
         const int segs = (int)std::min<size_t>(std::min(kUploadSegs, G), std::max<size_t>(1, xBytes / kSegBytes));
         SDB_CK(cudaEventRecord(segEv[kUploadSegs], st));  // Xin is free once the stream got here

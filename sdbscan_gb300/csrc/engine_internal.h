@@ -51,8 +51,10 @@ struct SweepSpec {
 //   [7] sng BF16 block failed (FP32 redoes it)   [8] a bounded wait of the plain distance kernel ran out
 constexpr int kErrSlots = 16;
 
-// Largest column copy of the packed distance tile (1M x 784 with D = 1024 and
-// m = 50 takes 0.33 GB).
+// Largest column copy of the packed distance tile, and most distances that a
+// sngOptics fit keeps between its passes: 3 % of the GPU's memory each.  A bound
+// on memory, not a line between two speeds: 1M x 784 with D = 1024 and m = 50
+// copies 0.33 GB, and sampled neighbourhoods copy as much as the data hold.
 constexpr size_t kMaxCandBytes = (size_t)8 << 30;
 
 struct sdb_engine {

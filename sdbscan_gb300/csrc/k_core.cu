@@ -344,8 +344,9 @@ __device__ __noinline__ int dedupe_sparse(const CoreArgs& a, DedupeWarp& sw, con
 // (Signatures per slot tested against the point's lists, the form before, walk
 // a candidate's lists where more than four hold it.  Core stage then and now:
 // 2K x 64, 51 lists a point, 317 -> 62 us; 50K x 128 328 -> 211; 1M x 784
-// 2147 -> 1744.)  Bound: L2 latency of the slot and list-mask loads, then
-// shared-memory wavefronts (61 % at 200K x 784).
+// 2147 -> 1744.)  Bound: latency, of the slot and list-mask loads in L2 and of
+// the shared-memory accesses in equal parts (5.5 stalled warps per issue each at
+// 200K x 784, issue slots 44 % and the shared-memory pipe 62 % used).
 __global__ void __launch_bounds__(128, 8) k_core_dedupe(CoreArgs a, int seenWords) {
     extern __shared__ __align__(16) unsigned char ddShm[];
     const int w = threadIdx.x >> 5;
