@@ -65,7 +65,7 @@ typedef struct {
     int32_t clusterNoise;         /* noiseClustering: 0, 1 (sDbscan-1NN), 2 (no-op) */
     float samplingProb;           /* prob: sDbscan-1NN core sampling; sng sample rate */
     int32_t verbose;              /* ver: print per-stage times                   */
-    int32_t n_threads;            /* numThreads: accepted for API parity, unused  */
+    int32_t n_threads;            /* numThreads: host threads of the OPTICS ordering, at most (<= 0: all) */
     int32_t random_seed;          /* randomSeed: < 0 means seeded from the clock  */
     int32_t precision;            /* sdb_precision                                */
 } sdb_params;

@@ -55,6 +55,8 @@ constexpr int kErrSlots = 16;
 // sngOptics fit keeps between its passes: 3 % of the GPU's memory each.  A bound
 // on memory, not a line between two speeds: 1M x 784 with D = 1024 and m = 50
 // copies 0.33 GB, and sampled neighbourhoods copy as much as the data hold.
+// Both stay for the next fit, like every buffer (8 GB allocated and freed again
+// takes 6 ms), unless a fit finds no memory (sdb_engine::fit).
 constexpr size_t kMaxCandBytes = (size_t)8 << 30;
 
 struct sdb_engine {

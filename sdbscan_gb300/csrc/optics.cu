@@ -276,9 +276,10 @@ sdb_status sdb_engine::optics_order(int64_t total) {
             }
         };
         // the largest floods first; a thread more for every 200K list entries
-        // (starting one takes 0.06 ms)
-        const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-        const size_t threads = std::min<size_t>({(size_t)hw, order.size(), (size_t)(kept / 200000) + 1, (size_t)32});
+        // (starting one takes 0.06 ms), and no more than the caller's n_threads
+        const unsigned most = prm.n_threads > 0 ? (unsigned)prm.n_threads
+                                                : std::max(1u, std::thread::hardware_concurrency());
+        const size_t threads = std::min<size_t>({(size_t)most, order.size(), (size_t)(kept / 200000) + 1, (size_t)32});
         std::vector<std::thread> helpers;
         try {
             for (size_t t = 1; t < threads; ++t) helpers.emplace_back(work);

@@ -92,3 +92,51 @@ def test_ordering_takes_the_distances_memory_when_there_is_no_other():
     got = fit(eps, cap)
     np.testing.assert_array_equal(got[0], order)
     np.testing.assert_array_equal(got[1], reach)
+
+
+@pytest.mark.parametrize("fit", ["soptics", "sngoptics"])
+def test_n_threads_bounds_the_orderings_host_threads(fit):
+    """n_threads = 1 runs the floods on the calling thread alone; the result is
+    the same with any number."""
+    import os
+    import threading
+
+    from sdbscan_gb300 import capi
+    n, d = 20000, 16
+    X = _clusters(n, d, 12, 0.35, 3, "mixed")
+
+    def run(n_threads):
+        e = capi.Engine(n, d)
+        e.set_params(n_proj=256, topK=8, topM=60, random_seed=4, n_threads=n_threads)
+        if fit == "sngoptics":
+            e.set_sng_params(samplingProb=0.03, random_seed=4, n_threads=n_threads)
+        call = e.fit_soptics if fit == "soptics" else e.fit_sngoptics
+        call(X, 0.06, 10)  # whatever the CUDA runtime starts is there now
+        stop = threading.Event()
+        seen = []
+
+        def watch():
+            while not stop.is_set():
+                seen.append(len(os.listdir("/proc/self/task")))
+
+        w = threading.Thread(target=watch)
+        w.start()
+        while not seen:
+            pass
+        before = seen[0]
+        for _ in range(5):
+            call(X, 0.06, 10)
+        stop.set()
+        w.join()
+        out = e.optics()
+        entries = int(e.core()[1].sum())
+        e.close()
+        return out, max(seen) - before, entries
+
+    one, extra, entries = run(1)
+    assert entries > 400000  # enough for helpers
+    assert extra == 0
+    for threads in (3, -1):
+        got, _, _ = run(threads)
+        np.testing.assert_array_equal(got[0], one[0])
+        np.testing.assert_array_equal(got[1], one[1])
