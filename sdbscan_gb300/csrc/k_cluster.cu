@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) k_union_tiles(ClusterArgs a) {
 __global__ void k_compress(ClusterArgs a) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n) return;
-    if (a.core[p]) a.parent[p] = find_root(a.parent, p);
+    if (a.core[p]) compress_point(a.parent, p);
 }
 
 // Border labels of one tile (parents are roots after k_compress).  A non-core

@@ -43,6 +43,11 @@ static __device__ int walk_root(const int32_t* parent, int x) {
     return x;
 }
 
+// p's parent becomes its root.  (Each thread writes its own point only: a walk
+// that halves paths would put an older ancestor over the root that another
+// thread has just written, and that point would take another cluster's label.)
+static __device__ void compress_point(int32_t* parent, int p) { parent[p] = walk_root(parent, p); }
+
 // The root a hooking round starts from: found by walking, or, where the paths
 // were compressed before the round (n >= kCompressRounds), the parent as it is.
 // carried: links of an earlier eps hold, whose edges the union pass does not

@@ -42,3 +42,11 @@ def test_the_orders_include_one_that_loses_a_link_beside_halved_paths(program):
     exe, _ = program
     r = _run(exe, 6, False)
     assert r.returncode == 1 and r.stdout.startswith("split:")
+
+
+def test_compression_leaves_every_point_at_its_root(program):
+    """Labels, borders and flood starts are read from the parents after it."""
+    exe, _ = program
+    r = subprocess.run([str(exe), "compress"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
+    assert re.match(r"\d+ cases", r.stdout)

@@ -12,6 +12,7 @@
 // united and no others (as k_union_tiles does in a carried round).  One set has
 // to be left.  Arguments: the point count that the hooking rule goes by, and 1
 // for a carried round's walk, 0 for the other rounds', which halves paths.
+// With one argument, compress_point instead (compress below).
 #include <setjmp.h>
 #include <ucontext.h>
 
@@ -151,7 +152,38 @@ static std::set<Mem> outcomes(const Mem& start) {
     return out;
 }
 
+// Compression of every forest on a path of the points (each parent smaller or
+// the point itself): every point of three has to end at its root.
+static int compress() {
+    long cases = 0;
+    for (int f = 0; f < 2 * 3 * 4 * 5; ++f) {
+        const Mem start{0, f % 2, f / 2 % 3, f / 6 % 4, f / 24, 5};
+        for (int skip = 0; skip < 5; ++skip) {  // three of points 1 to 4, or the last three
+            std::vector<int> points;
+            for (int i = 1; i < 5; ++i)
+                if (i != skip && (skip || i > 1)) points.push_back(i);
+            ++cases;
+            body = [&](int t) { compress_point(mem, points[t]); };
+            for (const Mem& end : outcomes(start))
+                for (int p : points) {
+                    int root = p;
+                    while (start[root] != root) root = start[root];
+                    if (end[p] == root) continue;
+                    std::printf("not at its root: %d of", p);
+                    for (int v : start) std::printf(" %d", v);
+                    std::printf(", at the end");
+                    for (int v : end) std::printf(" %d", v);
+                    std::printf("\n");
+                    return 1;
+                }
+        }
+    }
+    std::printf("%ld cases\n", cases);
+    return 0;
+}
+
 int main(int argc, char** argv) {
+    if (argc == 2) return compress();
     if (argc != 3) return 2;
     const int n = std::atoi(argv[1]);
     const bool carried = std::atoi(argv[2]) != 0;
